@@ -54,6 +54,39 @@ __device__ __forceinline__ float ld_dsmem(uint32_t addr) {
   return v;
 }
 
+// four consecutive fp32 values of one location in the C partial tiles of a cluster, added in rank order
+template <int C>
+__device__ __forceinline__ void sum_partials(uint32_t local_smem_addr, float (&y)[4]) {
+  float v[C][4];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const uint32_t a = C > 1 ? map_to_cta(local_smem_addr, static_cast<uint32_t>(c)) : local_smem_addr;
+    if (C > 1) asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c][0]), "=f"(v[c][1]), "=f"(v[c][2]), "=f"(v[c][3]) : "r"(a) : "memory");
+    else asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c][0]), "=f"(v[c][1]), "=f"(v[c][2]), "=f"(v[c][3]) : "r"(a) : "memory");
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    y[e] = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) y[e] += v[c][e];
+  }
+}
+__device__ __forceinline__ float2 unpack16(uint32_t w, int dtype) {
+  if (dtype == ORTB200_BF16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+__device__ __forceinline__ uint32_t pack16(float lo, float hi, int dtype) {
+  if (dtype == ORTB200_BF16) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float load16(const void* base, long long i, int dtype) {
+  return unpack16(static_cast<const uint16_t*>(base)[i], dtype).x;
+}
+
 // One 64-bit word carries a partial sum (low half) and the epoch of the launch that wrote it (high half).  A
 // naturally aligned 64-bit scalar access is single-copy atomic, so a reader that sees the expected epoch also sees
 // the value: no fence, no separate flag and no second NVLink round trip.
@@ -450,26 +483,33 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       // rows (a few KiB, L2 resident) and leave the factors in shared memory for the epilogue.
       pdl_wait_prior_grids();
       const int vecs = p.K / 8;
-      for (int j = q; j < BN; j += 4) {
+      // Only the token columns that this CTA finishes: every CTA of the cluster used to read all rows (40 tokens x 4096:
+      // 47 us for the qkv projection of 50 MB).  Eight loads per lane go out before the first is used.
+      for (int j = rank * (BN / C) + q; j < (rank + 1) * (BN / C); j += 4) {
         const int m = m0 + j;
         float ss = 0.f;
         if (m < m_end) {
           const uint4* row = reinterpret_cast<const uint4*>(static_cast<const uint8_t*>(p.x_rows) + static_cast<long long>(m) * p.K * 2);
-          for (int v = lane; v < vecs; v += 32) {
-            const uint4 u4 = __ldg(row + v);
-            const uint32_t w4[4] = {u4.x, u4.y, u4.z, u4.w};
+          for (int v0 = lane; v0 < vecs; v0 += 32 * 8) {
+            uint4 u[8];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float lo, hi;
-              if (p.dtype == ORTB200_BF16) {
-                lo = __uint_as_float(w4[e] << 16);
-                hi = __uint_as_float(w4[e] & 0xffff0000u);
-              } else {
-                const __half2 h2 = *reinterpret_cast<const __half2*>(&w4[e]);
-                lo = __low2float(h2);
-                hi = __high2float(h2);
+            for (int b = 0; b < 8; ++b) u[b] = v0 + 32 * b < vecs ? __ldg(row + v0 + 32 * b) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+              const uint32_t w4[4] = {u[b].x, u[b].y, u[b].z, u[b].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                float lo, hi;
+                if (p.dtype == ORTB200_BF16) {
+                  lo = __uint_as_float(w4[e] << 16);
+                  hi = __uint_as_float(w4[e] & 0xffff0000u);
+                } else {
+                  const __half2 h2 = *reinterpret_cast<const __half2*>(&w4[e]);
+                  lo = __low2float(h2);
+                  hi = __high2float(h2);
+                }
+                ss += lo * lo + hi * hi;
               }
-              ss += lo * lo + hi * hi;
             }
           }
         }
@@ -482,7 +522,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       if (p.status) atomicExch(p.status, kStatusTimeoutEpilogue);
     }
     tcgen05_fence_after();
-    if (!extra && C > 1) {
+    if (!extra) {
 #pragma unroll 1
       for (int c = 0; c < S::kCols; c += 16) {
         float v[16];
@@ -491,6 +531,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
         for (int j = 0; j < 16; ++j) part[(c + j) * kBM + r] = v[j];
       }
+      if (C == 1) asm volatile("bar.sync 2, 128;" ::: "memory");   // the four epilogue warps only
     }
   }
 
@@ -499,83 +540,100 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
   if (warp >= 2 && warp < 6) {
     const int q = warp & 3;
-    const int r = q * 32 + lane;
-    const int n = n0 + r;
-    const bool n_ok = n < p.N;
-    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     pdl_wait_prior_grids();  // out / residual may still be in use by the previous kernel
-    const float bias_v = (p.bias != nullptr && n_ok)
-                             ? (p.dtype == ORTB200_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[bias0 + n])
-                                                        : __half2float(reinterpret_cast<const __half*>(p.bias)[bias0 + n]))
-                             : 0.0f;
     // token columns this CTA finishes
     const int cols_per = BN / C;
     const int j_begin = rank * cols_per;
     const uint32_t part_addr = smem_u32(part);
     const bool fused_ar = p.world > 1;
-    unsigned int epoch = 0;
+    if (!fused_ar) {
+      // Warp q takes token columns q, q + 4, ... and lane l weight rows 4 l .. 4 l + 3: one 16-byte load per partial
+      // tile instead of four warps reading the same column 4 bytes at a time, and 8-byte stores.
+      const int n = n0 + 4 * lane;
+      float bias_v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (p.bias != nullptr && n + e < p.N) bias_v[e] = load16(p.bias, bias0 + n + e, p.dtype);
+      const bool vec = (((reinterpret_cast<uintptr_t>(p.out) | reinterpret_cast<uintptr_t>(p.residual)) & 7) == 0) &&
+                       ((p.ldo | (p.residual ? p.ldr : 0)) & 3) == 0 && n + 4 <= p.N;
+#pragma unroll 1
+      for (int j = j_begin + q; j < j_begin + cols_per; j += 4) {
+        const int m = m0 + j;
+        if (m >= m_end) break;
+        const uint32_t off = static_cast<uint32_t>((j * kBM + 4 * lane) * 4);
+        float y[4], u[4];
+        switch (C) {
+          case 1: sum_partials<1>(part_addr + off, y); break;
+          case 2: sum_partials<2>(part_addr + off, y); break;
+          case 4: sum_partials<4>(part_addr + off, y); break;
+          default: sum_partials<8>(part_addr + off, y); break;
+        }
+        if (DUAL) {
+          switch (C) {
+            case 1: sum_partials<1>(part_addr + off + BN * kBM * 4, u); break;
+            case 2: sum_partials<2>(part_addr + off + BN * kBM * 4, u); break;
+            case 4: sum_partials<4>(part_addr + off + BN * kBM * 4, u); break;
+            default: sum_partials<8>(part_addr + off + BN * kBM * 4, u); break;
+          }
+        }
+        const float row_scale = p.rms_eps > 0.f ? s_rstd[j] * p.alpha : p.alpha;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          y[e] = y[e] * row_scale + bias_v[e];
+          y[e] = DUAL ? gated_unit(p.gate, y[e], u[e] * row_scale) : act_apply(p.act, y[e]);
+        }
+        const long long o = m * p.ldo + n, ro = m * p.ldr + n;
+        if (vec) {
+          if (p.residual) {
+            const uint2 rr = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p.residual) + ro);
+            const float2 a = unpack16(rr.x, p.dtype), b = unpack16(rr.y, p.dtype);
+            y[0] += a.x; y[1] += a.y; y[2] += b.x; y[3] += b.y;
+          }
+          *reinterpret_cast<uint2*>(static_cast<uint16_t*>(p.out) + o) = make_uint2(pack16(y[0], y[1], p.dtype), pack16(y[2], y[3], p.dtype));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (n + e >= p.N) break;
+            if (p.residual) y[e] += load16(p.residual, ro + e, p.dtype);
+            static_cast<uint16_t*>(p.out)[o + e] = static_cast<uint16_t>(pack16(y[e], 0.f, p.dtype));
+          }
+        }
+      }
+    } else {
+    // fused all-reduce: thread r owns weight row r, so that the thread that pushed an element also gathers and finishes it
+    const int r = q * 32 + lane;
+    const int n = n0 + r;
+    const bool n_ok = n < p.N;
+    const float bias_v = (p.bias != nullptr && n_ok) ? load16(p.bias, bias0 + n, p.dtype) : 0.0f;
     unsigned int spin_limit = kPeerSpinLimit;
-    long long stage_base = 0;  // element offset of staging[epoch & 1][0][0]
-    if (fused_ar) {
-      epoch = *reinterpret_cast<volatile unsigned int*>(p.epoch) + 1;  // stable: the previous fused launch has completed
-      // word 2 of the workspace header overrides the polling limit (0 = default); failure-detection tests set a small
-      // one so that a peer that never answers costs milliseconds
-      const unsigned int lim = reinterpret_cast<volatile unsigned int*>(p.epoch)[2];
-      if (lim != 0) spin_limit = lim;
-      stage_base = static_cast<long long>(epoch & 1) * p.world * p.slot_elems;
-    }
+    // stable: the previous fused launch has completed
+    const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(p.epoch) + 1;
+    // word 2 of the workspace header overrides the polling limit (0 = default); failure-detection tests set a small
+    // one so that a peer that never answers costs milliseconds
+    const unsigned int lim = reinterpret_cast<volatile unsigned int*>(p.epoch)[2];
+    if (lim != 0) spin_limit = lim;
+    // element offset of staging[epoch & 1][0][0]
+    const long long stage_base = static_cast<long long>(epoch & 1) * p.world * p.slot_elems;
 #pragma unroll 1
     for (int jj = 0; jj < cols_per; ++jj) {
       const int j = j_begin + jj;
-      float v = 0.f, u = 0.f;
-      if (C > 1) {
-        for (int c = 0; c < C; ++c) {
-          const uint32_t base = map_to_cta(part_addr, static_cast<uint32_t>(c));
-          v += ld_dsmem(base + static_cast<uint32_t>((j * kBM + r) * 4));
-          if (DUAL) u += ld_dsmem(base + static_cast<uint32_t>(((BN + j) * kBM + r) * 4));
-        }
-      } else {
-        float t1[8];
-        tmem_ld_x8(t_lane + (j & ~7), t1);
-        tmem_ld_wait();
-        v = t1[j & 7];
-        if (DUAL) {
-          tmem_ld_x8(t_lane + BN + (j & ~7), t1);
-          tmem_ld_wait();
-          u = t1[j & 7];
-        }
+      float v = 0.f;
+      for (int c = 0; c < C; ++c) {
+        const uint32_t base = C > 1 ? map_to_cta(part_addr, static_cast<uint32_t>(c)) : part_addr;
+        v += ld_dsmem(base + static_cast<uint32_t>((j * kBM + r) * 4));
       }
       const int m = m0 + j;
-      if (fused_ar) {
-        // push this rank's partial sum to every rank (its own copy included); 128 lanes write 1 KiB contiguous
-        if (n_ok && m < m_end) {
-          const long long off = stage_base + static_cast<long long>(p.rank) * p.slot_elems + static_cast<long long>(m) * p.ldo + n;
-          for (int d = 0; d < p.world; ++d) {
-            const int dst_rank = (p.rank + d) % p.world;  // spread the first stores over the peers
-            st_packed_sys(reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(p.peers[dst_rank]) + p.staging_offset) + off,
-                          v * p.alpha, epoch);
-          }
-        }
-        continue;
-      }
+      // push this rank's partial sum to every rank (its own copy included); 128 lanes write 1 KiB contiguous
       if (n_ok && m < m_end) {
-        const float row_scale = p.rms_eps > 0.f ? s_rstd[j] * p.alpha : p.alpha;
-        float y = v * row_scale + bias_v;
-        if (DUAL) {
-          y = gated_unit(p.gate, y, u * row_scale);
-        } else {
-          y = act_apply(p.act, y);
-        }
-        if (p.dtype == ORTB200_BF16) {
-          if (p.residual) y += __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.residual)[m * p.ldr + n]);
-          reinterpret_cast<__nv_bfloat16*>(p.out)[m * p.ldo + n] = __float2bfloat16_rn(y);
-        } else {
-          if (p.residual) y += __half2float(reinterpret_cast<const __half*>(p.residual)[m * p.ldr + n]);
-          reinterpret_cast<__half*>(p.out)[m * p.ldo + n] = __float2half_rn(y);
+        const long long off = stage_base + static_cast<long long>(p.rank) * p.slot_elems + static_cast<long long>(m) * p.ldo + n;
+        for (int d = 0; d < p.world; ++d) {
+          const int dst_rank = (p.rank + d) % p.world;  // spread the first stores over the peers
+          st_packed_sys(reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(p.peers[dst_rank]) + p.staging_offset) + off,
+                        v * p.alpha, epoch);
         }
       }
     }
-    if (fused_ar) {
+    {
       // gather: the thread that pushed element (m, n) also finishes it, so no CTA-wide barrier is needed; it polls the
       // word of every source rank in its own copy of the staging area until the word carries this launch's epoch
       const unsigned long long* stage_local =
@@ -650,6 +708,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           *reinterpret_cast<volatile unsigned int*>(p.epoch) = epoch;
         }
       }
+    }
     }
   }
 
