@@ -451,9 +451,11 @@ class GemmSwiGLUKernel final : public OpKernel {
   void Compute(Ctx& ctx) const override {
     const at::Tensor& x = ctx.RequiredInput(0);
     at::Tensor x2 = Flatten2D(x);
-    if (x2.size(0) > 128 && I_ % 8 == 0) {
-      // Large M: the two-accumulator kernel is limited to 128-token tiles (tensor memory), which costs more than it
-      // saves; one plain GEMM over the stacked gate | up rows at 256-token tiles plus a streaming SwiGLU is faster.
+    const bool on_pairs = act_ != ORTB200_ACT_CLAMPED_SWIGLU && gated_.lead == 0 && ortb200_gemm_gated_pairs(static_cast<int>(x2.size(0)), static_cast<int>(I_));
+    if (x2.size(0) > 128 && I_ % 8 == 0 && !on_pairs) {
+      // Between the decode sizes and the CTA-pair kernel's: the two-accumulator kernel is limited to 128-token tiles (tensor
+      // memory), which costs more than it saves; one plain GEMM over the stacked gate | up rows at 256-token tiles plus a
+      // streaming SwiGLU is faster.
       at::Tensor gu = LaunchNormedGemm(ctx, x2, w_, 2 * I_, 0, at::Tensor(), at::Tensor(), ORTB200_ACT_NONE, 1.f, rms_eps_, unit_gamma_);
       const int64_t cols = gated_.lead + I_, esize = x2.element_size();
       at::Tensor y = at::empty({x2.size(0), cols}, x2.options());

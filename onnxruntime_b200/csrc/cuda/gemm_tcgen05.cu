@@ -888,6 +888,11 @@ extern "C" int64_t ortb200_gemm_workspace_bytes(int M, int N, int K, int act) {
   return need > 65536 ? need : 65536;
 }
 
+// At prompt size the gated unit is an epilogue of the CTA-pair kernel, under the same rule as the plain GEMM over 2 N rows.
+extern "C" int ortb200_gemm_gated_pairs(int M, int N) {
+  return M >= 512 && static_cast<long long>((M + 255) / 256) * ((N + 127) / 128) >= 60;
+}
+
 extern "C" int ortb200_gemm_last_config(int* bn, int* splits, int* stages) {
   if (bn) *bn = g_last_config.bn;
   if (splits) *splits = g_last_config.splits;
@@ -924,13 +929,18 @@ extern "C" int ortb200_gemm(const ortb200_gemm_args* a, ortb200_stream_t stream_
   // single-CTA kernel on 8192 x 6144 x 4096.  Needs at least most of a wave of 74 pairs to pay off.
   const long long tiles256 = static_cast<long long>((a->M + 255) / 256) * ((a->N + 255) / 256);
   if (a->alpha_dev != nullptr && !fp8) return -16;  // the device-side alpha factor exists in the fp8 kernel only
+  const bool gated_pair_ok = dual && a->in_dtype == 0 && a->act != ORTB200_ACT_CLAMPED_SWIGLU && a->world <= 1 && a->rms_eps <= 0.f && !a->bias && !a->residual;
+  if (gated_pair_ok && a->force_bn == 0 && a->force_splits == 0 && (a->force_tile_rows == 512 || (a->force_tile_rows == 0 && ortb200_gemm_gated_pairs(a->M, a->N)))) {
+    g_last_config = {256, 2, 5};
+    return launch_gemm_2cta(a, stream);
+  }
   const bool pair_ok = !dual && !q4 && a->rms_eps <= 0.f && !(fp8 && a->world > 1);  // fp8 operands run on the pair kernel too
   // world > 1 (row-parallel linear at prompt size): only the CTA-pair kernel has the epilogue that pushes the product
   // into the all-reduce scatter areas; the reduction kernel is launched right behind it
   if (a->force_tile_rows == 512 || (a->world > 1 && pair_ok) ||
       (a->force_tile_rows == 0 && a->force_bn == 0 && a->force_splits == 0 && pair_ok && a->M >= 512 && tiles256 >= 60)) {
     const int rc2 = launch_gemm_2cta(a, stream);
-    g_last_config = {256, 2, 5};
+    g_last_config = {256, 2, 6};
     return rc2;
   }
   if (a->world > 1) return -12;  // no fused all-reduce for this combination

@@ -116,7 +116,7 @@ int ortb200_gemm(const ortb200_gemm_args* args, ortb200_stream_t stream);
 //   out[r, :] = act(x[r, :] @ w[e]^T + bias[e]) for first_row <= r < end_row of every tile {e, first_row, end_row, -}.
 // Tiles cover at most tile_rows rows each.  tile_rows in {16, 32, 64}: one CTA per (weight tile, token tile), the
 // grid has max_tiles rows of CTAs and the CTAs beyond *num_tiles leave at once.  tile_rows in {128, 256}: the
-// persistent large-tile kernel walks the list (SWIGLU needs 128).  w is [num_experts * w_rows_per_expert, K]; with act == SWIGLU the gate rows
+// persistent large-tile kernels walk the list (SWIGLU and GEGLU with a bias need 128).  w is [num_experts * w_rows_per_expert, K]; with act == SWIGLU the gate rows
 // of expert e start at e * w_rows_per_expert and the up rows dual_offset rows later (N = rows of each half).
 typedef struct {
   const void* x;          // [rows, K]
@@ -204,6 +204,8 @@ int64_t ortb200_allgather_gemm_max_rows(int world, int K, int64_t symm_bytes);
 int64_t ortb200_allgather_gemm_area_offset(int64_t symm_bytes, int parity);
 int64_t ortb200_allgather_gemm_flag_offset(int src);
 // Number of kernels one ortb200_gemm call launches (always 1).
+// 1 when ortb200_gemm runs a gated unit (SWIGLU or GEGLU without bias and residual) of N features on CTA pairs
+int ortb200_gemm_gated_pairs(int M, int N);
 int ortb200_gemm_last_config(int* bn, int* splits, int* stages);
 
 // ---------------------------------------------------------------------------
