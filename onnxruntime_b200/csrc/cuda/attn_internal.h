@@ -22,6 +22,7 @@ struct AttnParams {
   const int* past_seqlens;
   int block_size, max_blocks, num_blocks;
   int chunk;             // > 0: keys of the query's own chunk only
+  int group_log2;        // attn_prefill.cu: log2 of the query heads of one key head that a CTA takes together
 };
 
 // Packed queries over a paged cache, softmax weights as the sum of two 16-bit terms (the caller has checked the arguments).
