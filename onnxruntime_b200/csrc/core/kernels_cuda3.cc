@@ -341,7 +341,8 @@ bool DecodeMask(const at::Tensor& m, int64_t B, int64_t T, at::Tensor* lengths, 
     return true;
   }
   if (m.dim() == 2 && m.size(0) == B && m.size(1) == T) {
-    *key_mask = m.ne(0).to(at::kInt).contiguous();
+    // the kernels ask whether an entry is 0: an int32 mask needs no pass of its own
+    *key_mask = m.scalar_type() == at::kInt ? m.contiguous() : m.ne(0).to(at::kInt).contiguous();
     return true;
   }
   return false;
@@ -812,7 +813,10 @@ void Reg(KernelRegistry& r, const std::string& domain, const std::string& op, st
 // EmbedLayerNormalization: gather of the three embedding rows + LayerNorm in one kernel.
 class EmbedLayerNormKernel final : public WithFallback {
  public:
-  explicit EmbedLayerNormKernel(const OpKernelInfo& info) : WithFallback(info) { eps_ = info.node.attr_f("epsilon", 1e-12f); }
+  explicit EmbedLayerNormKernel(const OpKernelInfo& info) : WithFallback(info) {
+    eps_ = info.node.attr_f("epsilon", 1e-12f);
+    from_gathers_ = info.node.attr_i("ortb200_from_gathers", 0) != 0;
+  }
   void Compute(Ctx& ctx) const override {
     const at::Tensor& ids = ctx.RequiredInput(0);
     const at::Tensor& word = ctx.RequiredInput(2);
@@ -833,7 +837,10 @@ class EmbedLayerNormKernel final : public WithFallback {
       pos_ids = ctx.Input(8);
       ok = id_ok(pos_ids) && pos_ids.dim() == 2 && pos_ids.size(1) == ids.size(1) && (pos_ids.size(0) == ids.size(0) || pos_ids.size(0) == 1);
     }
-    if (!ok) {
+    // positions that the fusion derived from the sequence length: the slice it replaced had no more rows than the table
+    if (from_gathers_ && ids.dim() == 2 && ids.size(1) > pos.size(0))
+      ORTB_THROW(INVALID_ARGUMENT, "EmbedLayerNormalization: sequence length ", ids.size(1), " exceeds the ", pos.size(0), " position embeddings");
+    if (!ok || (from_gathers_ && ids.numel() == 0)) {
       Fallback(ctx);
       return;
     }
@@ -861,6 +868,7 @@ class EmbedLayerNormKernel final : public WithFallback {
     a.position_broadcast = pos_ids.defined() && pos_ids.size(0) == 1 && B > 1 ? 1 : 0;
     a.epsilon = eps_;
     a.dtype = dt;
+    a.wrap_negative = from_gathers_ ? 1 : 0;
     a.status = ctx.session()->StatusWord().data_ptr<int>();
     CheckLaunch(ortb200_embed_layernorm(&a, ctx.cuda_stream()), "ortb200_embed_layernorm");
     ctx.session()->AddLaunches(1);
@@ -874,6 +882,7 @@ class EmbedLayerNormKernel final : public WithFallback {
 
  private:
   float eps_ = 1e-12f;
+  bool from_gathers_ = false;   // made by the fusion out of Gathers: their reading of ids, positions 0 .. S - 1
 };
 
 // MatMulBlockQuantizedFp8Weight: the fp8 weight with its per-block scales is expanded to the activation type once (at

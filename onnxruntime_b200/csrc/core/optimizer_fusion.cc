@@ -383,6 +383,32 @@ int AttentionFusion(PassContext& c) {
 }
 
 // ------------------------------------------------------- EmbedLayerNorm
+// Slice(0 .. P - 1, [0], [Shape(ids)[1]], axis of the row): the positions 0 .. S - 1 that an exporter derives from the
+// sequence length.  P has to cover the position table and to be above 1 (a single row would broadcast).
+bool DerivedPositions(Graph& g, const std::string& value, const std::string& ids, int64_t table_rows) {
+  auto ints = [&](const Node* n, size_t i, std::vector<int64_t>* out) {
+    const at::Tensor* t = n->has_input(i) ? g.GetConstant(n->inputs[i]) : nullptr;
+    if (!t || !at::isIntegralType(t->scalar_type(), false)) return false;
+    at::Tensor c = t->to(at::kCPU, at::kLong).reshape({-1}).contiguous();
+    out->assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+    return true;
+  };
+  const Node* sl = g.Producer(value);
+  if (!sl || !sl->domain.empty() || sl->op_type != "Slice" || !sl->has_input(3)) return false;
+  const at::Tensor* row = g.GetConstant(sl->inputs[0]);
+  if (!row || row->dim() > 2 || (row->dim() == 2 && row->size(0) != 1) || row->numel() != table_rows || table_rows < 2) return false;
+  at::Tensor r = row->to(at::kCPU, at::kLong).reshape({-1});
+  std::vector<int64_t> starts, axes, steps = {1}, index;
+  if (!at::equal(r, at::arange(r.numel(), r.options())) || !ints(sl, 1, &starts) || !ints(sl, 3, &axes)) return false;
+  if (sl->has_input(4) && !ints(sl, 4, &steps)) return false;
+  if (starts != std::vector<int64_t>{0} || steps != std::vector<int64_t>{1} || axes.size() != 1 || (axes[0] != row->dim() - 1 && axes[0] != -1)) return false;
+  const Node* n = g.Producer(sl->inputs[2]);
+  if (n && n->domain.empty() && n->op_type == "Unsqueeze") n = g.Producer(n->inputs[0]);
+  if (!n || !n->domain.empty() || n->op_type != "Gather" || n->attr_i("axis", 0) != 0 || !ints(n, 1, &index) || index != std::vector<int64_t>{1}) return false;
+  const Node* shape = g.Producer(n->inputs[0]);
+  return shape && shape->domain.empty() && shape->op_type == "Shape" && shape->inputs[0] == ids && shape->attr_i("start", 0) == 0;
+}
+
 int EmbedLayerNormFusion(PassContext& c) {
   Graph& g = c.g;
   int count = 0;
@@ -436,7 +462,10 @@ int EmbedLayerNormFusion(PassContext& c) {
       // position ids must be the default 0..S-1 row(s) when constant
       const at::Tensor* pids = g.GetConstant(pos->inputs[1]);
       std::string position_ids_input;
-      if (pids) {
+      const bool derived = !pids && DerivedPositions(g, pos->inputs[1], word->inputs[1], g.GetConstant(pos->inputs[0])->size(0));
+      if (derived) {
+        // the node's own default: no index tensor to build on the host and to upload on every run
+      } else if (pids) {
         at::Tensor pc = pids->to(at::kCPU, at::kLong);
         at::Tensor first = pc.dim() == 2 ? pc[0] : pc;
         if (!at::equal(first, at::arange(first.numel(), first.options()))) continue;
@@ -458,6 +487,7 @@ int EmbedLayerNormFusion(PassContext& c) {
       const std::string mask_out = g.UniqueName("embed_mask_index");
       Node* f = g.AddNode("EmbedLayerNormalization", ins, {ln->outputs[0], mask_out}, kMSDomain, g.UniqueName("EmbedLayerNorm"));
       f->set_attr_f("epsilon", ln->attr_f("epsilon", 1e-12f));
+      if (derived) f->set_attr_i("ortb200_from_gathers", 1);   // the GPU kernel then reads ids as Gather does
       g.RemoveNode(ln);
       for (Node* a : adds) g.RemoveNode(a);
       for (Node* ga : gathers) g.RemoveNode(ga);

@@ -194,6 +194,10 @@ __global__ void __launch_bounds__(128) embed_layernorm_kernel(const ortb200_embe
   int64_t wid = id_at(a.input_ids, tok);
   int64_t pid = a.position_ids ? id_at(a.position_ids, a.position_broadcast ? s : tok) : s;
   int64_t sid = (a.segment_ids && a.segment_emb) ? id_at(a.segment_ids, tok) : -1;
+  if (a.wrap_negative) {
+    if (wid < 0) wid += a.word_rows;
+    if (sid < 0 && a.segment_ids && a.segment_emb) sid = sid + a.seg_rows < 0 ? a.seg_rows : sid + a.seg_rows;
+  }
   // ids outside the tables read row 0 and flag the launch (the reference fails the run on such ids)
   if (wid < 0 || wid >= a.word_rows || pid < 0 || pid >= a.pos_rows || (sid >= a.seg_rows)) {
     if (a.status && threadIdx.x == 0) atomicExch(a.status, kStatusBadArgument);

@@ -249,6 +249,7 @@ typedef struct {
   float epsilon;
   int dtype;
   int* status;         // optional device int
+  int wrap_negative;   // 1: negative word and segment ids count from the end of their table, as Gather reads them
 } ortb200_embed_layernorm_args;
 int ortb200_embed_layernorm(const ortb200_embed_layernorm_args* args, ortb200_stream_t stream);
 
