@@ -66,6 +66,13 @@ int launch_gemm_grouped_2cta(const ortb200_gemm_grouped_args* a, cudaStream_t st
 // bn in {16, 32, 64}.  Returns 0 or a negative launch error; reports the cluster size and pipeline depth used.
 int launch_gemm_smallm(const ortb200_gemm_args* a, int bn, cudaStream_t stream, int* cluster_out, int* stages_out);
 
+// Cluster size (split of K) of a decode-shaped problem; `force` > 0 asks for one.
+int pick_cluster(int tiles, int num_kb, int bn, int force);
+
+// Packed 4-bit weights on warp-level tensor instructions, up to kQ4MaxTokens tokens (gemm_q4.cu).
+constexpr int kQ4MaxTokens = 16;
+int launch_gemm_q4(const ortb200_gemm_args* a, cudaStream_t stream, int* cluster_out, int* stages_out);
+
 #ifdef __CUDACC__
 // ---- epilogue store pass shared by the large-M GEMM kernels (device code)
 template <int ACT>

@@ -19,6 +19,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include "gemm_internal.h"
+#include "gemm_small_device.cuh"
 #include "ortb200_kernels.h"
 #include "ptx_sm100.cuh"
 #include "tensor_map.h"
@@ -34,59 +35,6 @@ constexpr int kThreads = 192;
 // four expansion warps on every SM sub-partition, so one warp's barrier waits and stores hide behind another's ALU work.
 constexpr int kThreadsNBits = 320;
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// address of the same shared-memory location in CTA `cta` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_t cta) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta));
-  return r;
-}
-__device__ __forceinline__ float ld_dsmem(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
-}
-
-// four consecutive fp32 values of one location in the C partial tiles of a cluster, added in rank order
-template <int C>
-__device__ __forceinline__ void sum_partials(uint32_t local_smem_addr, float (&y)[4]) {
-  float v[C][4];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const uint32_t a = C > 1 ? map_to_cta(local_smem_addr, static_cast<uint32_t>(c)) : local_smem_addr;
-    if (C > 1) asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c][0]), "=f"(v[c][1]), "=f"(v[c][2]), "=f"(v[c][3]) : "r"(a) : "memory");
-    else asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[c][0]), "=f"(v[c][1]), "=f"(v[c][2]), "=f"(v[c][3]) : "r"(a) : "memory");
-  }
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    y[e] = 0.f;
-#pragma unroll
-    for (int c = 0; c < C; ++c) y[e] += v[c][e];
-  }
-}
-__device__ __forceinline__ float2 unpack16(uint32_t w, int dtype) {
-  if (dtype == ORTB200_BF16) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-  return __half22float2(*reinterpret_cast<const __half2*>(&w));
-}
-__device__ __forceinline__ uint32_t pack16(float lo, float hi, int dtype) {
-  if (dtype == ORTB200_BF16) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-  }
-  const __half2 h = __floats2half2_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ float load16(const void* base, long long i, int dtype) {
-  return unpack16(static_cast<const uint16_t*>(base)[i], dtype).x;
-}
-
 // One 64-bit word carries a partial sum (low half) and the epoch of the launch that wrote it (high half).  A
 // naturally aligned 64-bit scalar access is single-copy atomic, so a reader that sees the expected epoch also sees
 // the value: no fence, no separate flag and no second NVLink round trip.
@@ -101,17 +49,6 @@ __device__ __forceinline__ unsigned long long ld_packed_sys(const unsigned long 
 }
 // about a second of polling at most; then the launch reports kStatusTimeoutPeer and finishes with what it has
 constexpr unsigned int kPeerSpinLimit = 1u << 22;
-
-__device__ __forceinline__ float act_apply(int act, float v) {
-  switch (act) {
-    case ORTB200_ACT_GELU: return gelu_erf_fast(v);
-    case ORTB200_ACT_FASTGELU: return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * v * (1.0f + 0.044715f * v * v)));
-    case ORTB200_ACT_RELU: return fmaxf(v, 0.0f);
-    case ORTB200_ACT_SILU: return v / (1.0f + __expf(-v));
-    case ORTB200_ACT_QUICKGELU: return v / (1.0f + __expf(-1.702f * v));
-    default: return v;
-  }
-}
 
 // NBITS: the weight tile arrives as packed 4-bit values (32 bytes per row and k-block, nibbles pre-arranged by
 // ortb200_nbits_prepack).  Eight warps expand it to 16-bit values and store them straight into tensor memory
@@ -825,6 +762,7 @@ int launch_gemm_smallm(const ortb200_gemm_args* a, int bn, cudaStream_t stream, 
       default: return -8;
     }
   }
+  if (a->in_dtype == ORTB200_Q4 && a->world <= 1 && a->M <= kQ4MaxTokens) return launch_gemm_q4(a, stream, cluster_out, stages_out);
   if (nbits) {
     switch (bn) {
       case 16: *stages_out = 12; return launch_small<16, 12, false, 1>(tw, tx, p, grid, stream, pdl);
