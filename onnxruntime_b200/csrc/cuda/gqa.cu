@@ -59,7 +59,7 @@ static bool prep_vectorised(const Args* a) {
 }
 
 // VEC: see prep_vectorised.  The kernel only moves bytes: 8192 tokens x 48 heads of 128 took 171 us pair by pair (2-byte
-// accesses), the 200 MB take 31 us at the copy rate.
+// accesses) and takes 34 us in vectors; the 200 MB need 31 at the copy rate.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) gqa_prep_kernel(const ortb200_gqa_prep_args a) {
   const int b = blockIdx.x / a.S, s = blockIdx.x % a.S;
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(128) gqa_decode_kernel(const DecodeParams p) {
     fa[g] = aa;
   }
 
-  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last);
+  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last, sm_acc);
 }
 
 
@@ -584,6 +584,7 @@ static int launch_decode(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
     if (splits > 32) splits = 32;
     if (splits < 1) splits = 1;
   }
+  if (splits > 2 * H) splits = 2 * H;   // the merge keeps two floats per split and head where [4][G][H] floats were
   const int tiles = a->B * a->Nk * gparts;
   const int64_t need = 65536 + static_cast<int64_t>(tiles) * splits * G * (H + 4) * 4;
   if (splits > 1 && (!a->workspace || a->workspace_bytes < need || tiles > 16384)) splits = 1;

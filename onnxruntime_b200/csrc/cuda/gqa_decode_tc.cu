@@ -6,7 +6,7 @@
 //   MMA 1  S^T[128 keys, 16]   = K_tile[128 keys, 128 dims] . Q[16 heads, 128 dims]^T       (both K-major)
 //   MMA 2  O^T[128 dims, 16]  += V_tile^T[128 dims, 128 keys] . P[16 heads, 128 keys]^T     (V MN-major)
 // One CTA owns (batch, kv head, key split) and serves every query head of the kv head (up to 16) as the N columns.
-// K/V tiles arrive by TMA (128-byte swizzle) through a 3-stage ring; thread t of the 4 softmax warps owns key t of
+// K/V tiles arrive by TMA (128-byte swizzle) through a ring of slots; thread t of the 4 softmax warps owns key t of
 // the tile (its TMEM lane of S^T): mask, scale, exponentiate, write the 16-bit probabilities into the swizzled
 // K-major layout MMA 2 reads.  The reference maximum of a head is only raised when a tile exceeds it by 2^8
 // (probabilities stay below 256), so O^T is rescaled in tensor memory a handful of times per sequence instead of
@@ -36,28 +36,36 @@ namespace ortb200 {
 namespace {
 
 constexpr int kTile = 128;                 // keys per tile
-constexpr int kStages = 3;
 constexpr int kBox = 128 * 128;            // [128 rows][64 elems] of 16-bit data
 constexpr int kTileBytes = 2 * kBox;       // K or V tile: two boxes (dims 0-63, 64-127)
-constexpr int kStageBytes = 2 * kTileBytes;
 constexpr int kQBox = 16 * 128;            // [16 heads][64 dims]
-constexpr int kOffQ = kStages * kStageBytes;
-constexpr int kOffP = kOffQ + 2 * kQBox;
-template <bool SPLIT>
+constexpr int kMaxSlots = 6;
+constexpr int kSms = 148;
+// K and V tiles alternate through one ring of slots.  Six slots: one CTA per SM, for grids that fit the machine once.  Three
+// slots: two CTAs share an SM with the same bytes in flight, and one's prologue, query rotation and merge of splits run while
+// the other streams.  40 sequences of 1000 - 4000 keys, 8 kv heads of 128, bf16: 101 -> 82 us (the bytes need 60); 32 of 1024 -
+// 4096, 8 heads per kv head: 90 -> 74 (47); one of 4096 in 16 splits: 30 -> 15 (mostly the merge).  (The remainders of SPLIT
+// take shared memory: always six.)
+template <bool SPLIT, int SLOTS>
 struct Smem {
+  static constexpr int kSlots = SLOTS;
+  static constexpr int kOffQ = kSlots * kTileBytes;
+  static constexpr int kOffP = kOffQ + 2 * kQBox;
   static constexpr int kPBox = (SPLIT ? 32 : 16) * 128;       // [16 heads, 16 remainders (SPLIT)][64 keys]
-  static constexpr int kOffMax = kOffP + 2 * 2 * kPBox;       // float [2][4][16]
+  static constexpr int kPBytes = 2 * 2 * kPBox, kXchBytes = 17 * 128 * 4;
+  static constexpr int kOffXch = kOffP;                       // float [17][128]: q heads and the new key, for the rotary partner (before the first P)
+  static constexpr int kOffMax = kOffP + (kPBytes > kXchBytes ? kPBytes : kXchBytes);   // float [2][4][16]
   static constexpr int kOffSum = kOffMax + 2 * 4 * 16 * 4;    // float [4][16]
-  static constexpr int kOffXch = kOffSum + 4 * 16 * 4;        // float [17][128]: q heads and the new key, for the rotary partner
-  static constexpr int kOffNew = kOffXch + 17 * 128 * 4;      // float [16]: scores of the new key
+  static constexpr int kOffNew = kOffSum + 4 * 16 * 4;        // float [16]: scores of the new key
   static constexpr int kOffBar = kOffNew + 16 * 4;
   static constexpr int kBytes = kOffBar + 256 + 1024;
+  static_assert(kBytes * (SLOTS == 3 ? 2 : 1) <= 226 * 1024, "shared memory");
 };
-constexpr int kThreads = 160;              // 4 softmax warps + 1 TMA / MMA warp
+constexpr int kThreads = 192;              // 4 softmax warps, an MMA warp, a TMA warp
 constexpr int kTmemCols = 64;              // S^T buffers at columns 0 and 16, O^T at 32, its remainders at 48
 constexpr float kRaise = 8.f;              // raise the reference maximum only past 2^8
 
-enum { BAR_Q = 0, BAR_FULL0, BAR_EMPTY0 = BAR_FULL0 + kStages, BAR_S0 = BAR_EMPTY0 + kStages, BAR_S1, BAR_P0, BAR_P1, BAR_O,
+enum { BAR_Q = 0, BAR_FULL0, BAR_EMPTY0 = BAR_FULL0 + kMaxSlots, BAR_S0 = BAR_EMPTY0 + kMaxSlots, BAR_S1, BAR_P0, BAR_P1, BAR_O,
        BAR_END, BAR_COUNT };
 
 __device__ __forceinline__ float redux_max(float v) {
@@ -81,12 +89,13 @@ __device__ __forceinline__ void tmem_ld_heads(uint32_t taddr, float* v) {
   tmem_ld_wait();
 }
 
-template <typename T, int G, bool PAGED, bool SPLIT>
-__global__ void __launch_bounds__(kThreads, 1)
+template <typename T, int G, bool PAGED, bool SPLIT, int SLOTS>
+__global__ void __launch_bounds__(kThreads, SLOTS == 3 ? 2 : 1)
 gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const DecodeParams p, const int piece_rows) {
-  using L = Smem<SPLIT>;
+  using L = Smem<SPLIT, SLOTS>;
   constexpr int H = 128;
+  constexpr int kSlots = L::kSlots;
   constexpr int GV = (G + 7) / 8 * 8;   // columns fetched from tensor memory
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   extern __shared__ uint8_t smem_raw[];
@@ -145,7 +154,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int k_end = owns_new ? total - 1 : min(total, k_begin + chunk);
   const int n_tiles = k_end > k_begin ? (k_end - k_begin + kTile - 1) / kTile : 0;
 
-  if (warp == 4 && p.prefetch != nullptr) {
+  if (warp == 5 && p.prefetch != nullptr) {
     // This grid moves a few tens of MB and leaves most of the memory bandwidth idle: ask the L2 for this CTA's slice
     // of the next kernel's weights now, so that kernel finds them on chip.
     const long long cta = (static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
@@ -156,31 +165,27 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       bulk_prefetch_l2(p.prefetch + off, static_cast<uint32_t>(nbytes));
     }
   }
-  if (warp == 4) {
-    // ------------------------------------------------------------ TMA producer + MMA issuer (lane 0 issues; with a
-    // paged cache lane i fetches piece i of a tile)
-    const uint32_t idesc_s = umma_idesc_f16(kBf16, kTile, 16);
-    const uint32_t idesc_o = umma_idesc_f16(kBf16, H, SPLIT ? 32 : 16) | (1u << 15);   // A (= V^T) is MN-major
-    const uint32_t q_addr = smem_u32(smem + kOffQ);
+  // load i is the K tile (i even) or the V tile (i odd) of key tile i / 2, in slot i % kSlots
+  if (warp == 5) {
+    // ------------------------------------------------------------ TMA producer (with a paged cache lane i fetches piece i)
     const int pieces = PAGED ? kTile / piece_rows : 1;
-    auto load_tile = [&](int t) {
-      const int s = t % kStages;
-      uint8_t* st = smem + s * kStageBytes;
-      const int key0 = k_begin + t * kTile;
+    bool ok = true;
+    for (int i = 0; i < 2 * n_tiles; ++i) {
+      const int s = i % kSlots, key0 = k_begin + (i >> 1) * kTile;
+      if (i >= kSlots && !mbar_wait(&bars[BAR_EMPTY0 + s], ((i / kSlots) - 1) & 1)) { ok = false; break; }
+      uint8_t* dst = smem + s * kTileBytes;
+      const CUtensorMap* tm = (i & 1) ? &tm_v : &tm_k;
       if (!PAGED) {
         if (lane == 0) {
-          mbar_expect_tx(&bars[BAR_FULL0 + s], kStageBytes);
+          mbar_expect_tx(&bars[BAR_FULL0 + s], kTileBytes);
           const int plane = b * p.Nk + kvh;
 #pragma unroll
-          for (int bx = 0; bx < 2; ++bx) {
-            tma_load_3d(st + bx * kBox, &tm_k, &bars[BAR_FULL0 + s], bx * 64, key0, plane);
-            tma_load_3d(st + kTileBytes + bx * kBox, &tm_v, &bars[BAR_FULL0 + s], bx * 64, key0, plane);
-          }
+          for (int bx = 0; bx < 2; ++bx) tma_load_3d(dst + bx * kBox, tm, &bars[BAR_FULL0 + s], bx * 64, key0, plane);
         }
       } else {
         // pieces whose first key lies beyond the range are not fetched (their block-table entries may be unset)
         const int live = min(pieces, (k_end - key0 + piece_rows - 1) / piece_rows);
-        if (lane == 0) mbar_expect_tx(&bars[BAR_FULL0 + s], static_cast<uint32_t>(live) * piece_rows * 4 * 128);
+        if (lane == 0) mbar_expect_tx(&bars[BAR_FULL0 + s], static_cast<uint32_t>(live) * piece_rows * 2 * 128);
         __syncwarp();
         if (lane < live) {
           const int key = key0 + lane * piece_rows;
@@ -188,18 +193,23 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const int blk = bi < p.max_blocks ? p.block_table[static_cast<long long>(b) * p.max_blocks + bi] : -1;
           // a block index outside the pool reads as zeros (TMA fills out-of-range rows)
           const int row = blk >= 0 ? blk * p.block_size + key % p.block_size : 0x3fffff00;
-          uint8_t* dst = st + lane * piece_rows * 128;
 #pragma unroll
-          for (int bx = 0; bx < 2; ++bx) {
-            tma_load_3d(dst + bx * kBox, &tm_k, &bars[BAR_FULL0 + s], bx * 64, row, kvh);
-            tma_load_3d(dst + kTileBytes + bx * kBox, &tm_v, &bars[BAR_FULL0 + s], bx * 64, row, kvh);
-          }
+          for (int bx = 0; bx < 2; ++bx) tma_load_3d(dst + lane * piece_rows * 128 + bx * kBox, tm, &bars[BAR_FULL0 + s], bx * 64, row, kvh);
         }
       }
       __syncwarp();
-    };
+    }
+    if (!ok && lane == 0 && p.status) atomicExch(p.status, kStatusTimeoutProducer);
+  } else if (warp == 4) {
+    // ------------------------------------------------------------ MMA issuer: the whole warp waits, lane 0 issues (a lone
+    // lane that polled the barriers made every launch 2.7 us longer)
+    const uint32_t idesc_s = umma_idesc_f16(kBf16, kTile, 16);
+    const uint32_t idesc_o = umma_idesc_f16(kBf16, H, SPLIT ? 32 : 16) | (1u << 15);   // A (= V^T) is MN-major
+    const uint32_t q_addr = smem_u32(smem + L::kOffQ);
+    auto full = [&](int i) { return mbar_wait(&bars[BAR_FULL0 + i % kSlots], (i / kSlots) & 1); };
     auto issue_s = [&](int t) {
-      const uint32_t k_addr = smem_u32(smem + (t % kStages) * kStageBytes);
+      const int slot = (2 * t) % kSlots;
+      const uint32_t k_addr = smem_u32(smem + slot * kTileBytes);
       const uint32_t d = tmem_base + (t & 1) * 16;
 #pragma unroll
       for (int kk = 0; kk < H / 16; ++kk) {
@@ -207,50 +217,45 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                  umma_desc_sw128(q_addr + (kk / 4) * kQBox + (kk % 4) * 32), idesc_s, kk > 0 ? 1u : 0u);
       }
       umma_commit(&bars[BAR_S0 + (t & 1)]);
+      umma_commit(&bars[BAR_EMPTY0 + slot]);
     };
     bool ok = true;
     if (n_tiles > 0) {
       if (lane == 0 && !fused) {
         mbar_expect_tx(&bars[BAR_Q], 2 * kQBox);
-        tma_load_3d(smem + kOffQ, &tm_q, &bars[BAR_Q], 0, head0, b);
-        tma_load_3d(smem + kOffQ + kQBox, &tm_q, &bars[BAR_Q], 64, head0, b);
+        tma_load_3d(smem + L::kOffQ, &tm_q, &bars[BAR_Q], 0, head0, b);
+        tma_load_3d(smem + L::kOffQ + kQBox, &tm_q, &bars[BAR_Q], 64, head0, b);
       }
-      const int pre = n_tiles < kStages ? n_tiles : kStages;
-      for (int t = 0; t < pre; ++t) load_tile(t);
-      ok = mbar_wait(&bars[BAR_Q], 0) && mbar_wait(&bars[BAR_FULL0], 0);
+      ok = mbar_wait(&bars[BAR_Q], 0) && full(0);
       if (ok && lane == 0) {
         tcgen05_fence_after();
         issue_s(0);
       }
       for (int t = 0; t < n_tiles && ok; ++t) {
-        const int s = t % kStages;
         if (t + 1 < n_tiles) {
           // S^T buffer (t + 1) & 1 was consumed before P of tile t - 1 was published, which this warp waited for
-          if (!mbar_wait(&bars[BAR_FULL0 + (t + 1) % kStages], ((t + 1) / kStages) & 1)) { ok = false; break; }
+          if (!full(2 * t + 2)) { ok = false; break; }
           if (lane == 0) {
             tcgen05_fence_after();
             issue_s(t + 1);
           }
         }
-        if (!mbar_wait(&bars[BAR_P0 + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
+        if (!full(2 * t + 1) || !mbar_wait(&bars[BAR_P0 + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
         if (lane == 0) {
           tcgen05_fence_after();
-          const uint32_t v_addr = smem_u32(smem + s * kStageBytes + kTileBytes);
-          const uint32_t p_addr = smem_u32(smem + kOffP + (t & 1) * 2 * L::kPBox);
+          const int slot = (2 * t + 1) % kSlots;
+          const uint32_t v_addr = smem_u32(smem + slot * kTileBytes);
+          const uint32_t p_addr = smem_u32(smem + L::kOffP + (t & 1) * 2 * L::kPBox);
 #pragma unroll
           for (int kk = 0; kk < kTile / 16; ++kk) {
             umma_f16(tmem_o, umma_desc_mn_sw128(v_addr + kk * 2048, kBox, 1024),
                      umma_desc_sw128(p_addr + (kk / 4) * L::kPBox + (kk % 4) * 32), idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
           }
-          umma_commit(&bars[BAR_EMPTY0 + s]);
+          umma_commit(&bars[BAR_EMPTY0 + slot]);
           umma_commit(&bars[BAR_O]);
           if (t == n_tiles - 1) umma_commit(&bars[BAR_END]);
         }
         __syncwarp();
-        if (t + kStages < n_tiles) {
-          if (!mbar_wait(&bars[BAR_EMPTY0 + s], (t / kStages) & 1)) { ok = false; break; }
-          load_tile(t + kStages);
-        }
       }
       if (!ok && lane == 0 && p.status) atomicExch(p.status, kStatusTimeoutMma);
     }
@@ -302,7 +307,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const T k_t = from_float<T>(kx);
     float part[G];
     {
-      uint8_t* qb = smem + kOffQ + (t >> 6) * kQBox;
+      uint8_t* qb = smem + L::kOffQ + (t >> 6) * kQBox;
       const int col = t & 63;
 #pragma unroll
       for (int g = 0; g < 16; ++g) {
@@ -399,7 +404,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
       }
       // probabilities of this key for every head, rounded to the MMA input type (the sum uses what enters MMA 2)
-      uint8_t* pb = smem + kOffP + (t & 1) * 2 * L::kPBox + (tid >> 6) * L::kPBox;
+      uint8_t* pb = smem + L::kOffP + (t & 1) * 2 * L::kPBox + (tid >> 6) * L::kPBox;
       const int col = tid & 63;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
@@ -413,9 +418,9 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (k_begin + (t + 1) * kTile > k_end) {
         // last, partial tile: rows past the range hold whatever the cache (or an earlier tile) left there; a
         // non-finite value times a zero probability would poison MMA 2, so those V rows are cleared
-        if (ok && !mbar_wait(&bars[BAR_FULL0 + t % kStages], (t / kStages) & 1)) ok = false;
+        if (ok && !mbar_wait(&bars[BAR_FULL0 + (2 * t + 1) % kSlots], ((2 * t + 1) / kSlots) & 1)) ok = false;
         if (!valid) {
-          uint8_t* vrow = smem + (t % kStages) * kStageBytes + kTileBytes + tid * 128;
+          uint8_t* vrow = smem + ((2 * t + 1) % kSlots) * kTileBytes + tid * 128;
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             *reinterpret_cast<uint4*>(vrow + i * 16) = make_uint4(0, 0, 0, 0);
@@ -494,22 +499,23 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
   }
   const int tile = b * p.Nk + kvh;
-  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last);
+  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last, reinterpret_cast<float*>(smem));
 }
 
-template <typename T, int G, bool PAGED, bool SPLIT>
+template <typename T, int G, bool PAGED, bool SPLIT, int SLOTS>
 int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p, int piece_rows,
               dim3 grid, cudaStream_t stream, bool use_pdl) {
-  auto kern = gqa_decode_tc_kernel<T, G, PAGED, SPLIT>;
+  auto kern = gqa_decode_tc_kernel<T, G, PAGED, SPLIT, SLOTS>;
+  constexpr int kBytes = Smem<SPLIT, SLOTS>::kBytes;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<SPLIT>::kBytes) != cudaSuccess) return -10;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess) return -10;
     attr_set = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = Smem<SPLIT>::kBytes;
+  cfg.dynamicSmemBytes = kBytes;
   cfg.stream = stream;
   cudaLaunchAttribute attrs[1];
   if (use_pdl) {
@@ -521,12 +527,25 @@ int launch_tc(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
   return cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, p, piece_rows) == cudaSuccess ? 0 : -11;
 }
 
-template <typename T, bool PAGED, bool SPLIT>
+template <typename T, bool PAGED, bool SPLIT, int SLOTS>
 int launch_tc_g(int group, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DecodeParams& p,
                 int piece_rows, dim3 grid, cudaStream_t stream, bool use_pdl) {
-  if (group <= 4) return launch_tc<T, 4, PAGED, SPLIT>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
-  if (group <= 8) return launch_tc<T, 8, PAGED, SPLIT>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
-  return launch_tc<T, 16, PAGED, SPLIT>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
+  if (group <= 4) return launch_tc<T, 4, PAGED, SPLIT, SLOTS>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
+  if (group <= 8) return launch_tc<T, 8, PAGED, SPLIT, SLOTS>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
+  return launch_tc<T, 16, PAGED, SPLIT, SLOTS>(tq, tk, tv, p, piece_rows, grid, stream, use_pdl);
+}
+
+// one CTA per SM while the grid fits the machine once, else two
+template <typename T>
+int launch_tc_t(const ortb200_gqa_decode_args* a, int group, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
+                const DecodeParams& p, int piece_rows, dim3 grid, cudaStream_t stream, bool pdl) {
+  if (a->split_weights) return launch_tc_g<T, true, true, kMaxSlots>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
+  const bool shared_sm = static_cast<long long>(grid.x) * grid.y * grid.z > kSms;
+  if (a->block_table)
+    return shared_sm ? launch_tc_g<T, true, false, 3>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl)
+                     : launch_tc_g<T, true, false, kMaxSlots>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
+  return shared_sm ? launch_tc_g<T, false, false, 3>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl)
+                   : launch_tc_g<T, false, false, kMaxSlots>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
 }
 
 }  // namespace
@@ -555,19 +574,25 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   const int base = a->B * a->Nk;
   int splits = a->splits;
   if (splits <= 0) {
-    // One CTA per SM at most.  Merging splits costs about as much as four tiles, so a grid that already covers a
+    // Small grids: one CTA per SM at most.  Merging splits costs about as much as four tiles, so a grid that already covers a
     // good part of the machine with short key ranges is not split; otherwise at least two tiles per split.
+    // Grids of more than half the machine: two or three splits of at least ten tiles even out unequal lengths (20 sequences of
+    // 750 - 3000 keys, 8 kv heads: 51 us in one piece, 41 in two; 40 of 1000 - 4000: 87 and, in three, 82; 64 of 250 - 1000
+    // would lose, 43 and 51).
     // a chunk may begin within a tile
     const int tiles = a->chunk > 0 && a->chunk < a->Smax - kTile ? (a->chunk + kTile - 1) / kTile + 1 : (a->Smax + kTile - 1) / kTile;
     if (base >= 32 && tiles <= 12) {
       splits = 1;
+    } else if (base > kSms / 2) {
+      splits = tiles >= 30 ? 3 : tiles >= 20 ? 2 : 1;
     } else {
-      splits = 148 / base;
+      splits = kSms / base;
       if (splits > (tiles + 1) / 2) splits = (tiles + 1) / 2;
       if (splits > 32) splits = 32;
       if (splits < 1) splits = 1;
     }
   }
+  if (splits > 256) splits = 256;   // the merge keeps two floats per split and head in the slots
   if (base > 16384) return -4;
   while (splits > 1 && 65536 + static_cast<int64_t>(base) * splits * G * (H + 4) * 4 > a->workspace_bytes) --splits;
   if (a->workspace_bytes < 65536) return -4;
@@ -617,14 +642,8 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
     p.prefetch_per_cta = static_cast<int>(((bytes + ctas - 1) / ctas + 15) & ~15LL);
   }
   const bool pdl = a->use_pdl != 0;
-  if (a->dtype == ORTB200_BF16) {
-    if (a->split_weights) return launch_tc_g<__nv_bfloat16, true, true>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
-    return a->block_table ? launch_tc_g<__nv_bfloat16, true, false>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl)
-                          : launch_tc_g<__nv_bfloat16, false, false>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
-  }
-  if (a->split_weights) return launch_tc_g<__half, true, true>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
-  return a->block_table ? launch_tc_g<__half, true, false>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl)
-                        : launch_tc_g<__half, false, false>(group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
+  return a->dtype == ORTB200_BF16 ? launch_tc_t<__nv_bfloat16>(a, group, tq, tk, tv, p, piece_rows, grid, stream, pdl)
+                                  : launch_tc_t<__half>(a, group, tq, tk, tv, p, piece_rows, grid, stream, pdl);
 }
 
 }  // namespace ortb200

@@ -53,22 +53,26 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream);
 // unnormalised output (fa), and every thread holds the running maximum (fm, natural-log domain) and the sum of
 // exponentials (fl) of the CTA's key range.  With splits > 1 the state goes to the workspace and the CTA that
 // arrives last on the tile's counter merges all splits; that CTA (or the only one) normalises and stores.
+// `scratch`: 2 * splits * G floats of shared memory that nothing else needs any more.  In the merge a thread owns four dims of
+// one head and fetches eight splits at a time, after all threads have fetched the maxima and sums: a dim per thread, head
+// after head and load after load, was a chain of 2 * splits * G L2 round trips.
 template <typename T, int H, int G>
 __device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, int split, int b, int head0, int n_heads,
                                               int tid, float (&fm)[G], float (&fl)[G], float (&fa)[G],
-                                              unsigned int* sm_last_ptr) {
+                                              unsigned int* sm_last_ptr, float* scratch) {
   const bool owner = tid < H;
   unsigned int& sm_last = *sm_last_ptr;
   bool finalize = true;
   if (p.splits > 1) {
-    // publish partial state: ws[tile][split][g][H + 2]
-    float* my = p.ws + ((static_cast<size_t>(tile) * p.splits + split) * G) * (H + 2);
+    // publish partial state: ws[tile][split][g][H + 4]
+    constexpr int kState = H + 4;   // rows of 16-byte vectors
+    float* my = p.ws + ((static_cast<size_t>(tile) * p.splits + split) * G) * kState;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-      if (owner) my[g * (H + 2) + tid] = fa[g];
+      if (owner) my[g * kState + tid] = fa[g];
       if (tid == 0) {
-        my[g * (H + 2) + H] = fm[g];
-        my[g * (H + 2) + H + 1] = fl[g];
+        my[g * kState + H] = fm[g];
+        my[g * kState + H + 1] = fl[g];
       }
     }
     __threadfence();
@@ -80,24 +84,47 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, i
       sm_last = last;
     }
     __syncthreads();
-    finalize = sm_last != 0;
-    if (finalize) {
+    finalize = false;   // the merge below stores the result itself
+    if (sm_last != 0) {
       __threadfence();
-      const float* base = p.ws + (static_cast<size_t>(tile) * p.splits * G) * (H + 2);
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
+      const float* base = p.ws + (static_cast<size_t>(tile) * p.splits * G) * kState;
+      const int states = p.splits * G;
+      for (int i = tid; i < states; i += blockDim.x) {
+        scratch[i] = __ldcg(&base[i * kState + H]);
+        scratch[states + i] = __ldcg(&base[i * kState + H + 1]);
+      }
+      __syncthreads();
+      for (int i = tid; i < n_heads * (H / 4); i += blockDim.x) {
+        const int g = i / (H / 4), d = i % (H / 4) * 4;
         float mm = kNegBig;
-        for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, __ldcg(&base[(s * G + g) * (H + 2) + H]));
-        float ll = 0.f, aa = 0.f;
-        for (int s = 0; s < p.splits; ++s) {
-          const float* ps = base + (s * G + g) * (H + 2);
-          const float c = safe_exp_diff(__ldcg(&ps[H]), mm);
-          ll += __ldcg(&ps[H + 1]) * c;
-          if (owner) aa += __ldcg(&ps[tid]) * c;
+        for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, scratch[s * G + g]);
+        float ll = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s0 = 0; s0 < p.splits; s0 += 8) {
+          float4 v[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            v[e] = s0 + e < p.splits ? __ldcg(reinterpret_cast<const float4*>(&base[((s0 + e) * G + g) * kState + d])) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (s0 + e >= p.splits) break;
+            const float c = safe_exp_diff(scratch[(s0 + e) * G + g], mm);
+            ll += scratch[states + (s0 + e) * G + g] * c;
+            acc[0] += v[e].x * c;
+            acc[1] += v[e].y * c;
+            acc[2] += v[e].z * c;
+            acc[3] += v[e].w * c;
+          }
         }
-        fm[g] = mm;
-        fl[g] = ll;
-        fa[g] = aa;
+        float scale = 1.f;
+        if (p.head_sink) {
+          const float sink = to_float<T>(static_cast<const T*>(p.head_sink)[head0 + g]);
+          const float m2 = fmaxf(mm, sink);
+          scale = safe_exp_diff(mm, m2);
+          ll = ll * scale + __expf(sink - m2);
+        }
+        T* o = static_cast<T*>(p.out) + b * p.out_ld + static_cast<long long>(head0 + g) * H + d;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = from_float<T>(ll > 0.f ? acc[e] * scale / ll : 0.f);
       }
     }
   }
