@@ -810,6 +810,28 @@ void Reg(KernelRegistry& r, const std::string& domain, const std::string& op, st
 
 }  // namespace
 
+// Cast to e4m3 of 16-bit activations in front of the fp8 GEMMs; every other Cast keeps its kernel.
+class CastE4m3Kernel final : public WithFallback {
+ public:
+  explicit CastE4m3Kernel(const OpKernelInfo& info) : WithFallback(info) {}
+  void Compute(Ctx& ctx) const override {
+    if (ctx.InputIsString(0)) {
+      Fallback(ctx);
+      return;
+    }
+    const at::Tensor& x = ctx.RequiredInput(0);
+    const int dt = x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16 ? DtypeCode(x.scalar_type()) : -1;
+    if (dt < 0 || !x.is_cuda() || !x.is_contiguous() || x.numel() == 0 || (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15)) {
+      Fallback(ctx);
+      return;
+    }
+    at::Tensor y = at::empty(x.sizes(), x.options().dtype(at::kFloat8_e4m3fn));
+    CheckLaunch(ortb200_cast_e4m3(x.data_ptr(), y.data_ptr(), x.numel(), dt, ctx.cuda_stream()), "ortb200_cast_e4m3");
+    ctx.session()->AddLaunches(1);
+    ctx.SetOutput(0, y);
+  }
+};
+
 // EmbedLayerNormalization: gather of the three embedding rows + LayerNorm in one kernel.
 class EmbedLayerNormKernel final : public WithFallback {
  public:
@@ -1002,6 +1024,7 @@ void RegisterCudaKernels3(KernelRegistry& r) {
   Reg<MoeKernel>(r, MS, "ShardedMoE");
   Reg<MoeKernel>(r, MS, "QMoE");
   Reg<GemmFloat8Kernel>(r, MS, "GemmFloat8");
+  Reg<CastE4m3Kernel>(r, "", "Cast", {}, [](const Node& n, const Graph&) { return n.attr_i("to", 1) == pb::FLOAT8E4M3FN; });
   Reg<BlockFp8WeightMatMulKernel>(r, MS, "MatMulBlockQuantizedFp8Weight");
   Reg<EmbedLayerNormKernel>(r, MS, "EmbedLayerNormalization");
   Reg<SymmCollectiveKernel>(r, MS, "AllReduce");

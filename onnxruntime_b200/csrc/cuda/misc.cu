@@ -133,6 +133,49 @@ __global__ void __launch_bounds__(256) swiglu_vec8_kernel(const uint4* __restric
   pdl_launch_dependents();
 }
 
+// 16-bit -> e4m3 bytes, two vectors of eight elements a thread; bound by the 3 bytes an element moves.  7608 x 4096: 16.0 us (14 at
+// the copy rate), with the tensor library's conversion 24.7; 7608 x 1024: 5.2 against 7.4.
+template <bool BF16>
+__device__ __forceinline__ uint32_t e4m3_pair(uint32_t w) {
+  float lo, hi;
+  uint16_t r;
+  if (BF16) {
+    lo = __uint_as_float(w << 16);
+    hi = __uint_as_float(w & 0xffff0000u);
+    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
+  } else {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    lo = f.x;
+    hi = f.y;
+    asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(r) : "r"(w));
+  }
+  uint32_t v = r;
+  // the sign as the 32-bit value has it: converting an fp16 NaN drops it
+  if (!(fabsf(lo) <= 464.f)) v = (v & 0xff00u) | 0x7fu | ((__float_as_uint(lo) >> 24) & 0x80u);
+  if (!(fabsf(hi) <= 464.f)) v = (v & 0x00ffu) | 0x7f00u | ((__float_as_uint(hi) >> 16) & 0x8000u);
+  return v;
+}
+template <bool BF16>
+__global__ void __launch_bounds__(256) cast_e4m3_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ y, int64_t n) {
+  pdl_wait_prior_grids();
+  const int64_t first = (static_cast<int64_t>(blockIdx.x) * 512 + threadIdx.x) * 8;
+  uint4 v[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (first + u * 2048 + 8 <= n) v[u] = __ldg(reinterpret_cast<const uint4*>(x + first + u * 2048));
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int64_t i = first + u * 2048;
+    if (i + 8 <= n) {
+      *reinterpret_cast<uint2*>(y + i) =
+          make_uint2(e4m3_pair<BF16>(v[u].x) | (e4m3_pair<BF16>(v[u].y) << 16), e4m3_pair<BF16>(v[u].z) | (e4m3_pair<BF16>(v[u].w) << 16));
+    } else {
+      for (int64_t j = i; j < n; ++j) y[j] = static_cast<uint8_t>(e4m3_pair<BF16>(x[j]));
+    }
+  }
+  pdl_launch_dependents();
+}
+
 template <typename T>
 __global__ void rotary_kernel(const T* __restrict__ x, T* __restrict__ y, const int64_t* __restrict__ position_ids,
                               int64_t position_offset, const T* __restrict__ cos_cache, const T* __restrict__ sin_cache,
@@ -246,6 +289,18 @@ static int launch_gated_unit(const void* x, void* y, int64_t rows, int cols, int
     swiglu_kernel<__half, GELU><<<g, 256, 0, st>>>(static_cast<const __half*>(x), static_cast<__half*>(y), rows, cols);
   else if (dtype == ORTB200_F32)
     swiglu_kernel<float, GELU><<<g, 256, 0, st>>>(static_cast<const float*>(x), static_cast<float*>(y), rows, cols);
+  else return -4;
+  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+extern "C" int ortb200_cast_e4m3(const void* x, void* y, int64_t n, int dtype, ortb200_stream_t stream_) {
+  cudaStream_t st = static_cast<cudaStream_t>(stream_);
+  if (!x || !y || n <= 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(y) & 7)) return -3;
+  const int64_t blocks = (n + 4095) / 4096;
+  if (blocks > 0x7fffffff) return -9;
+  if (dtype == ORTB200_BF16) cast_e4m3_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n);
+  else if (dtype == ORTB200_F16) cast_e4m3_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n);
   else return -4;
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
