@@ -81,6 +81,9 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const float* v) {
                : "memory");
 }
 
+// Bounded wait of a whole warp: all lanes go on, or all give up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
 // G query heads live in columns [0, G) of S^T and O^T; columns are read eight at a time
 template <int G>
 __device__ __forceinline__ void tmem_ld_heads(uint32_t taddr, float* v) {
@@ -172,7 +175,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     bool ok = true;
     for (int i = 0; i < 2 * n_tiles; ++i) {
       const int s = i % kSlots, key0 = k_begin + (i >> 1) * kTile;
-      if (i >= kSlots && !mbar_wait(&bars[BAR_EMPTY0 + s], ((i / kSlots) - 1) & 1)) { ok = false; break; }
+      if (i >= kSlots && !mbar_wait_warp(&bars[BAR_EMPTY0 + s], ((i / kSlots) - 1) & 1)) { ok = false; break; }
       uint8_t* dst = smem + s * kTileBytes;
       const CUtensorMap* tm = (i & 1) ? &tm_v : &tm_k;
       if (!PAGED) {
@@ -206,7 +209,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t idesc_s = umma_idesc_f16(kBf16, kTile, 16);
     const uint32_t idesc_o = umma_idesc_f16(kBf16, H, SPLIT ? 32 : 16) | (1u << 15);   // A (= V^T) is MN-major
     const uint32_t q_addr = smem_u32(smem + L::kOffQ);
-    auto full = [&](int i) { return mbar_wait(&bars[BAR_FULL0 + i % kSlots], (i / kSlots) & 1); };
+    auto full = [&](int i) { return mbar_wait_warp(&bars[BAR_FULL0 + i % kSlots], (i / kSlots) & 1); };
     auto issue_s = [&](int t) {
       const int slot = (2 * t) % kSlots;
       const uint32_t k_addr = smem_u32(smem + slot * kTileBytes);
@@ -226,7 +229,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tma_load_3d(smem + L::kOffQ, &tm_q, &bars[BAR_Q], 0, head0, b);
         tma_load_3d(smem + L::kOffQ + kQBox, &tm_q, &bars[BAR_Q], 64, head0, b);
       }
-      ok = mbar_wait(&bars[BAR_Q], 0) && full(0);
+      ok = mbar_wait_warp(&bars[BAR_Q], 0) && full(0);
       if (ok && lane == 0) {
         tcgen05_fence_after();
         issue_s(0);
@@ -240,7 +243,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             issue_s(t + 1);
           }
         }
-        if (!full(2 * t + 1) || !mbar_wait(&bars[BAR_P0 + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
+        if (!full(2 * t + 1) || !mbar_wait_warp(&bars[BAR_P0 + (t & 1)], (t >> 1) & 1)) { ok = false; break; }
         if (lane == 0) {
           tcgen05_fence_after();
           const int slot = (2 * t + 1) % kSlots;
