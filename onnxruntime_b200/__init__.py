@@ -17,6 +17,7 @@ _here = _os.path.dirname(_os.path.abspath(__file__))
 _built = any(f.startswith("_core") and f.endswith(".so") for f in _os.listdir(_here))
 
 if _built:
+    globals().pop("__getattr__", None)   # a module that was imported before the build keeps its names through a reload
     import torch as _torch  # noqa: F401  (loads libtorch before the extension)
 
     from .capi import *  # noqa: F401,F403
