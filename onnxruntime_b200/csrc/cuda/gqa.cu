@@ -586,13 +586,15 @@ static int launch_decode(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   }
   if (splits > 2 * H) splits = 2 * H;   // the merge keeps two floats per split and head where [4][G][H] floats were
   const int tiles = a->B * a->Nk * gparts;
-  const int64_t need = 65536 + static_cast<int64_t>(tiles) * splits * G * (H + 4) * 4;
-  if (splits > 1 && (!a->workspace || a->workspace_bytes < need || tiles > 16384)) splits = 1;
+  const int64_t need = static_cast<int64_t>(tiles) * splits * G * (H + 4) * 4;
+  int64_t state_bytes = 0;
+  float* const states = decode_states(a, &state_bytes);
+  if (splits > 1 && (state_bytes < need || tiles > 16384)) splits = 1;
   DecodeParams p;
   p.q = a->q; p.k_cache = a->k_cache; p.v_cache = a->v_cache; p.seqlens_k = a->seqlens_k; p.head_sink = a->head_sink;
   p.out = a->out;
   p.counters = reinterpret_cast<unsigned int*>(a->workspace);
-  p.ws = a->workspace ? reinterpret_cast<float*>(static_cast<char*>(a->workspace) + 65536) : nullptr;
+  p.ws = states;
   p.status = a->status;
   p.B = a->B; p.N = a->N; p.Nk = a->Nk; p.Smax = a->Smax; p.splits = splits; p.window = a->window; p.gparts = gparts;
   p.scale = a->scale != 0.f ? a->scale : 1.0f / sqrtf(static_cast<float>(H));

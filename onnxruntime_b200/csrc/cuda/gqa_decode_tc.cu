@@ -597,7 +597,9 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   }
   if (splits > 256) splits = 256;   // the merge keeps two floats per split and head in the slots
   if (base > 16384) return -4;
-  while (splits > 1 && 65536 + static_cast<int64_t>(base) * splits * G * (H + 4) * 4 > a->workspace_bytes) --splits;
+  int64_t state_bytes = 0;
+  float* const states = decode_states(a, &state_bytes);
+  while (splits > 1 && static_cast<int64_t>(base) * splits * G * (H + 4) * 4 > state_bytes) --splits;
   if (a->workspace_bytes < 65536) return -4;
 
   const CUtensorMapDataType dt = a->dtype == ORTB200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -624,7 +626,7 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   p.q = a->q; p.k_cache = a->k_cache; p.v_cache = a->v_cache; p.seqlens_k = a->seqlens_k; p.head_sink = a->head_sink;
   p.out = a->out;
   p.counters = reinterpret_cast<unsigned int*>(a->workspace);
-  p.ws = reinterpret_cast<float*>(static_cast<char*>(a->workspace) + 65536);
+  p.ws = states;
   p.status = a->status;
   p.B = a->B; p.N = a->N; p.Nk = a->Nk; p.Smax = a->Smax; p.splits = splits; p.window = a->window; p.gparts = 1;
   p.scale = a->scale != 0.f ? a->scale : 1.0f / sqrtf(static_cast<float>(H));

@@ -45,6 +45,14 @@ __device__ __forceinline__ float safe_exp_diff(float a, float b) {
 }
 
 
+// Where the states of the splits lie behind the counters, and how many bytes there are: the merge reads 16-byte vectors, and a
+// caller's workspace need only be aligned for floats.
+inline float* decode_states(const ortb200_gqa_decode_args* a, int64_t* bytes) {
+  const uintptr_t ws = reinterpret_cast<uintptr_t>(a->workspace), first = (ws + 65536 + 15) & ~uintptr_t(15);
+  *bytes = ws ? a->workspace_bytes - static_cast<int64_t>(first - ws) : 0;
+  return ws ? reinterpret_cast<float*>(first) : nullptr;
+}
+
 // tcgen05 decode kernel (gqa_decode_tc.cu)
 bool gqa_decode_tc_supported(const ortb200_gqa_decode_args* a);
 int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream);
