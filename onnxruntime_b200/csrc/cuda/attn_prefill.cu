@@ -15,6 +15,8 @@
 // 128: 250 -> 122 us; 64 x 384 masked, 16 heads of 64: 286 -> 115 us; 2284 packed tokens of 25 sequences, 20 of them single
 // tokens: 206 -> 91 us.  2 x 4096 causal reaches 877 TFLOP/s; at 8 x 1024 (9 tiles a CTA) the special-function units are
 // 31 % busy: what is left is the latency of a CTA's first loads and last stores.
+// Value rows behind the last visible key (of a cache, or of a masked tail) may hold anything and never reach the product.  Rows
+// that a key mask hides in front of that key take part with weight 0 and have to be finite.
 // (attn_split.cu holds the form whose softmax weights stay 32-bit up to the product with V.)
 //
 // Replaces, for prompt processing and encoder self-attention, the FlashAttention-2
@@ -61,7 +63,7 @@ __device__ __forceinline__ unsigned key_keep_bits(const int* key_mask, int b, in
 }
 
 enum { BAR_Q = 0, BAR_K_FULL, BAR_K_EMPTY = BAR_K_FULL + 3, BAR_V_FULL = BAR_K_EMPTY + 3, BAR_V_EMPTY = BAR_V_FULL + 3, BAR_S = BAR_V_EMPTY + 3,
-       BAR_P = BAR_S + 2, BAR_O = BAR_P + 2, BAR_END, BAR_COUNT };
+       BAR_P = BAR_S + 2, BAR_O = BAR_P + 2, BAR_END, BAR_V_LAST, BAR_COUNT };
 
 
 template <int HD>
@@ -130,15 +132,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   const int total = paged ? p.past_seqlens[b] + S : (p.seqlens_k ? p.seqlens_k[b] + 1 : p.kv_len);
   const int past = paged ? total - S : (p.first_prompt ? 0 : total - S);
-  // key range needed by this query tile
-  int kv_end = total;
-  if (p.causal) kv_end = min(kv_end, past + q0 + tq);
-  kv_end = min(kv_end, p.kv_len);
+  int visible_end = min(total, p.kv_len);
   if (mask_kept) {   // nothing is visible behind the last unmasked key
     int end = 0;
     for (int w = 0; w < kAttnThreads / 32; ++w) end = max(end, mask_end[w]);
-    kv_end = min(kv_end, end);
+    visible_end = min(visible_end, end);
   }
+  // key range needed by this query tile
+  const int kv_end = p.causal ? min(visible_end, past + q0 + tq) : visible_end;
   int kv_begin = 0;
   if (p.window > 0) kv_begin = max(0, past + q0 - p.window + 1) / kKT * kKT;
   if (p.chunk > 0) kv_begin = max(kv_begin, (past + q0) / p.chunk * p.chunk / kKT * kKT);
@@ -146,10 +147,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
 
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
+      const int live = visible_end - kv_begin - (n_tiles - 1) * kKT;   // rows of the last value tile that belong to keys, when below 64
       mbar_expect_tx(&bars[BAR_Q], L::kBoxes * L::kQBox);
       for (int bx = 0; bx < L::kBoxes; ++bx)
         for (int h = 0; h < (1 << p.group_log2); ++h)   // rows of a head behind those of the head before it
           tma_load_4d(smem + bx * L::kQBox + h * tq * 128, &tm_q, &bars[BAR_Q], bx * 64, q_row0 + q0, head0 + h, paged ? 0 : b);
+      const int cleared = live < kKT ? n_tiles - 1 : -1;   // the tile whose other rows are cleared
       bool ok = true;
       int s = 0;
       uint32_t parity = 1;   // the first round over the stages waits for nothing
@@ -167,8 +170,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
         mbar_expect_tx(&bars[BAR_K_FULL + s], L::kBoxes * L::kBox);
         for (int bx = 0; bx < L::kBoxes; ++bx) tma_load_4d(st + bx * L::kBox, &tm_k, &bars[BAR_K_FULL + s], bx * 64, c1, kvh, c3);
         if (!mbar_wait(&bars[BAR_V_EMPTY + s], parity)) { ok = false; break; }
-        mbar_expect_tx(&bars[BAR_V_FULL + s], L::kBoxes * L::kBox);
-        for (int bx = 0; bx < L::kBoxes; ++bx) tma_load_4d(st + (L::kBoxes + bx) * L::kBox, &tm_v, &bars[BAR_V_FULL + s], bx * 64, c1, kvh, c3);
+        uint64_t* v_bar = &bars[t == cleared ? BAR_V_LAST : BAR_V_FULL + s];
+        mbar_expect_tx(v_bar, L::kBoxes * L::kBox);
+        for (int bx = 0; bx < L::kBoxes; ++bx) tma_load_4d(st + (L::kBoxes + bx) * L::kBox, &tm_v, v_bar, bx * 64, c1, kvh, c3);
+        if (t == cleared) ok = clear_stale_rows<L::kBoxes, L::kBox>(st + L::kBoxes * L::kBox, live, v_bar, &bars[BAR_V_FULL + s]);
         if (++s == STAGES) { s = 0; parity ^= 1u; }
       }
       if (!ok && p.status) atomicExch(p.status, kStatusTimeoutProducer);

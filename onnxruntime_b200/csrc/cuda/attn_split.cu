@@ -48,7 +48,7 @@ struct Smem {
 };
 
 enum { BAR_Q = 0, BAR_K_FULL, BAR_K_EMPTY = BAR_K_FULL + 2, BAR_V_FULL = BAR_K_EMPTY + 2, BAR_V_EMPTY = BAR_V_FULL + 2, BAR_S = BAR_V_EMPTY + 2,
-       BAR_P = BAR_S + 2, BAR_O = BAR_P + 2, BAR_END, BAR_COUNT };
+       BAR_P = BAR_S + 2, BAR_O = BAR_P + 2, BAR_END, BAR_V_LAST, BAR_COUNT };
 
 template <int KB, int VB, int STAGES, bool LATENT>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -118,6 +118,8 @@ attn_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (LATENT && bx >= sp.plain_boxes) tma_load_4d(smem + bx * L::kQBox, &tm_qr, &bars[BAR_Q], (bx - sp.plain_boxes) * 64, q_row0 + q0, head, 0);
         else tma_load_4d(smem + bx * L::kQBox, &tm_q, &bars[BAR_Q], bx * 64, q_row0 + q0, head, 0);
       }
+      const int live = total - kv_begin - (n_tiles - 1) * kKT;   // rows of the last value tile that belong to keys, when below 64
+      const int cleared = live < kKT ? n_tiles - 1 : -1;   // the tile whose other rows are cleared
       bool ok = true;
       for (int t = 0; t < n_tiles && ok; ++t) {
         const int s = t % STAGES, parity = (t / STAGES - 1) & 1, key0 = kv_begin + t * kKT;
@@ -138,8 +140,10 @@ attn_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             tma_load_4d(st + bx * L::kBox, &tm_k, &bars[BAR_K_FULL + s], bx * 64, c1, kvh, c3);
         }
         if (t >= STAGES && !mbar_wait(&bars[BAR_V_EMPTY + s], parity)) { ok = false; break; }
-        mbar_expect_tx(&bars[BAR_V_FULL + s], VB * L::kBox);
-        for (int bx = 0; bx < VB; ++bx) tma_load_4d(st + (KB + bx) * L::kBox, &tm_v, &bars[BAR_V_FULL + s], bx * 64, c1, kvh, c3);
+        uint64_t* v_bar = &bars[t == cleared ? BAR_V_LAST : BAR_V_FULL + s];
+        mbar_expect_tx(v_bar, VB * L::kBox);
+        for (int bx = 0; bx < VB; ++bx) tma_load_4d(st + (KB + bx) * L::kBox, &tm_v, v_bar, bx * 64, c1, kvh, c3);
+        if (t == cleared) ok = clear_stale_rows<VB, L::kBox>(st + KB * L::kBox, live, v_bar, &bars[BAR_V_FULL + s]);
       }
       if (!ok && p.status) atomicExch(p.status, kStatusTimeoutProducer);
     }

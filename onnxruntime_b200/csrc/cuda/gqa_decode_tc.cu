@@ -81,9 +81,6 @@ __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const float* v) {
                : "memory");
 }
 
-// Bounded wait of a whole warp: all lanes go on, or all give up.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
-
 // G query heads live in columns [0, G) of S^T and O^T; columns are read eight at a time
 template <int G>
 __device__ __forceinline__ void tmem_ld_heads(uint32_t taddr, float* v) {

@@ -164,7 +164,7 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
       const int live = (min(kTile, k_end - key0) + kGranule - 1) / kGranule;   // granules
       const int pieces = live * granule_pieces;   // at most 16: lanes take a piece of one of two boxes each
       const int sub = lane / pieces, piece = lane - sub * pieces, key = key0 + piece * p.piece_rows;
-      // blocks outside the sequence or the pool are clamped: masked keys only have to be finite
+      // blocks outside the sequence or the pool are clamped: masked keys may hold anything (see below)
       const int bi = min(key / p.block_size, p.max_blocks - 1);
       const int blk = min(max(p.block_table[static_cast<long long>(b) * p.max_blocks + bi], 0), p.num_blocks - 1);
       const int row = blk * p.block_size + key % p.block_size;
@@ -199,6 +199,17 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
         umma_commit(&bars[BAR_S]);
       }
       __syncwarp();
+      if (k_end - key0 < live * kGranule) {
+        // loaded rows behind the sequence: 0 * NaN would reach MMA 2, so they are cleared once MMA 1 has read the tile
+        if (!mbar_wait_warp(&bars[BAR_S], i & 1)) { ok = false; break; }
+#pragma unroll 1
+        for (int j = (k_end - key0) * 8 + lane; j < live * kGranule * 8; j += 32) {
+#pragma unroll 1
+          for (int bx = 0; bx < p.wide_boxes; ++bx) *reinterpret_cast<uint4*>(smem + bx * kBox + j * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async();
+        __syncwarp();
+      }
       if (!mbar_wait(&bars[BAR_P], i & 1)) { ok = false; break; }
       if (lane == 0) {
         tcgen05_fence_after();

@@ -94,6 +94,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// Bounded wait of a whole warp: all lanes go on, or all give up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
 // --------------------------------------------------------------------- TMA
 // 2-D tiled load, global -> shared, completion counted in bytes on `bar`.
 // (x = innermost coordinate in elements; x * elem_size must be 16-byte aligned)
