@@ -195,6 +195,9 @@ void RegisterQOrderedKernels(KernelRegistry& r);
 void RegisterStringKernels(KernelRegistry& r);
 // Cast with a string on either side (kernels_string.cc); false when neither side is a string
 bool CastWithStrings(OpKernelContext& ctx, int32_t to);
+// x in a float-8 type.  saturate: what lies beyond the largest number becomes it, infinities too; otherwise it becomes NaN (an
+// infinity in E5M2).  NaN stays NaN.
+at::Tensor ToFloat8(const at::Tensor& x, at::ScalarType type, bool saturate);
 void RegisterControlFlowKernels(KernelRegistry& r);
 void RegisterCollectiveKernels(KernelRegistry& r);
 void RegisterHybridKernels(KernelRegistry& r);

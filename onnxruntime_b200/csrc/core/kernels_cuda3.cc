@@ -813,7 +813,7 @@ void Reg(KernelRegistry& r, const std::string& domain, const std::string& op, st
 // Cast to e4m3 of 16-bit activations in front of the fp8 GEMMs; every other Cast keeps its kernel.
 class CastE4m3Kernel final : public WithFallback {
  public:
-  explicit CastE4m3Kernel(const OpKernelInfo& info) : WithFallback(info) {}
+  explicit CastE4m3Kernel(const OpKernelInfo& info) : WithFallback(info) { saturate_ = info.node.attr_i("saturate", 1) != 0; }
   void Compute(Ctx& ctx) const override {
     if (ctx.InputIsString(0)) {
       Fallback(ctx);
@@ -826,10 +826,13 @@ class CastE4m3Kernel final : public WithFallback {
       return;
     }
     at::Tensor y = at::empty(x.sizes(), x.options().dtype(at::kFloat8_e4m3fn));
-    CheckLaunch(ortb200_cast_e4m3(x.data_ptr(), y.data_ptr(), x.numel(), dt, ctx.cuda_stream()), "ortb200_cast_e4m3");
+    CheckLaunch(ortb200_cast_e4m3(x.data_ptr(), y.data_ptr(), x.numel(), dt, saturate_ ? 1 : 0, ctx.cuda_stream()), "ortb200_cast_e4m3");
     ctx.session()->AddLaunches(1);
     ctx.SetOutput(0, y);
   }
+
+ private:
+  bool saturate_ = true;
 };
 
 // EmbedLayerNormalization: gather of the three embedding rows + LayerNorm in one kernel.

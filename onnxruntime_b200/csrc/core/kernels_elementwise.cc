@@ -16,7 +16,7 @@ namespace {
 using Ctx = OpKernelContext;
 constexpr int kMax = 1 << 30;
 
-at::Tensor CastTo(const at::Tensor& x, int32_t onnx_type) {
+at::Tensor CastTo(const at::Tensor& x, int32_t onnx_type, bool saturate) {
   const at::ScalarType st = ToTorchType(onnx_type);
   if (x.scalar_type() == st) return x;
   if (st == at::kBool) return x.ne(0);
@@ -24,6 +24,7 @@ at::Tensor CastTo(const at::Tensor& x, int32_t onnx_type) {
     // float -> int truncates toward zero; go through int64 for unsigned targets
     return at::trunc(x.to(at::kDouble)).to(at::kLong).to(st);
   }
+  if (c10::isFloat8Type(st)) return ToFloat8(x, st, saturate);
   return x.to(st);
 }
 
@@ -37,6 +38,13 @@ at::Tensor VariadicReduce(Ctx& ctx, const std::function<at::Tensor(const at::Ten
 at::Tensor Gelu(const at::Tensor& x, bool tanh_approx) { return at::gelu(x, tanh_approx ? "tanh" : "none"); }
 
 }  // namespace
+
+at::Tensor ToFloat8(const at::Tensor& x, at::ScalarType type, bool saturate) {
+  if (!saturate || x.scalar_type() == type) return x.to(type);
+  const double largest = type == at::kFloat8_e4m3fn ? 448.0 : type == at::kFloat8_e4m3fnuz ? 240.0 : 57344.0;
+  const bool wide = x.scalar_type() == at::kDouble || x.scalar_type() == at::kHalf || x.scalar_type() == at::kBFloat16;
+  return at::clamp(wide ? x : x.to(at::kFloat), -largest, largest).to(type);
+}
 
 #define ORTB_UNARY(NAME, SINCE, EXPR)                                                   \
   r.RegisterFn("", NAME, SINCE, kMax, [](Ctx& ctx) {                                    \
@@ -145,12 +153,12 @@ void RegisterElementwiseKernels(KernelRegistry& r) {
   r.RegisterFn("", "Cast", 1, kMax, [](Ctx& ctx) {
     const int32_t to = static_cast<int32_t>(ctx.node().attr_i("to", 1));
     if (CastWithStrings(ctx, to)) return;
-    ctx.SetOutput(0, CastTo(ctx.RequiredInput(0), to));
+    ctx.SetOutput(0, CastTo(ctx.RequiredInput(0), to, ctx.node().attr_i("saturate", 1) != 0));
   });
   r.RegisterFn("", "CastLike", 15, kMax, [](Ctx& ctx) {
     const int32_t to = ctx.InputIsString(1) ? static_cast<int32_t>(pb::STRING) : ToOnnxType(ctx.RequiredInput(1).scalar_type());
     if (CastWithStrings(ctx, to)) return;
-    ctx.SetOutput(0, CastTo(ctx.RequiredInput(0), to));
+    ctx.SetOutput(0, CastTo(ctx.RequiredInput(0), to, ctx.node().attr_i("saturate", 1) != 0));
   });
   r.RegisterFn("", "Dropout", 1, kMax, [](Ctx& ctx) {
     // inference: identity, mask of ones

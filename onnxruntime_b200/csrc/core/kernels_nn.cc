@@ -327,7 +327,7 @@ void QuantizeLinearImpl(Ctx& ctx) {
   }
   at::Tensor q = x.to(at::kFloat) / scale;
   if (c10::isFloat8Type(out_t)) {
-    ctx.SetOutput(0, q.to(out_t));
+    ctx.SetOutput(0, ToFloat8(q, out_t, n.attr_i("saturate", 1) != 0));
     return;
   }
   q = at::round(q);

@@ -295,7 +295,8 @@ bool CastWithStrings(OpKernelContext& ctx, int32_t to) {
       v.data_ptr<double>()[i] = std::strtod(t.c_str(), &end);
       ORTB_ENFORCE_ARG(end != t.c_str() && *end == '\0', "Cast: '", s[i], "' is not a number");
     }
-    ctx.SetOutput(0, v.to(ToTorchType(to)).to(x.device()));
+    const at::ScalarType type = ToTorchType(to);
+    ctx.SetOutput(0, (c10::isFloat8Type(type) ? ToFloat8(v, type, ctx.node().attr_i("saturate", 1) != 0) : v.to(type)).to(x.device()));
     return true;
   }
   const bool integral = !x.is_floating_point();

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) swiglu_vec8_kernel(const uint4* __restric
 // 16-bit -> e4m3 bytes, two vectors of eight elements a thread; bound by the 3 bytes an element moves.  7608 x 4096: 16.0 us (14 at
 // the copy rate), with the tensor library's conversion 24.7; 7608 x 1024: 5.2 against 7.4.
 template <bool BF16>
-__device__ __forceinline__ uint32_t e4m3_pair(uint32_t w) {
+__device__ __forceinline__ uint32_t e4m3_pair(uint32_t w, float limit) {   // NaN beyond `limit`
   float lo, hi;
   uint16_t r;
   if (BF16) {
@@ -151,12 +151,12 @@ __device__ __forceinline__ uint32_t e4m3_pair(uint32_t w) {
   }
   uint32_t v = r;
   // the sign as the 32-bit value has it: converting an fp16 NaN drops it
-  if (!(fabsf(lo) <= 464.f)) v = (v & 0xff00u) | 0x7fu | ((__float_as_uint(lo) >> 24) & 0x80u);
-  if (!(fabsf(hi) <= 464.f)) v = (v & 0x00ffu) | 0x7f00u | ((__float_as_uint(hi) >> 16) & 0x8000u);
+  if (!(fabsf(lo) <= limit)) v = (v & 0xff00u) | 0x7fu | ((__float_as_uint(lo) >> 24) & 0x80u);
+  if (!(fabsf(hi) <= limit)) v = (v & 0x00ffu) | 0x7f00u | ((__float_as_uint(hi) >> 16) & 0x8000u);
   return v;
 }
 template <bool BF16>
-__global__ void __launch_bounds__(256) cast_e4m3_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ y, int64_t n) {
+__global__ void __launch_bounds__(256) cast_e4m3_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ y, int64_t n, float limit) {
   pdl_wait_prior_grids();
   const int64_t first = (static_cast<int64_t>(blockIdx.x) * 512 + threadIdx.x) * 8;
   uint4 v[2];
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(256) cast_e4m3_kernel(const uint16_t* __restri
     const int64_t i = first + u * 2048;
     if (i + 8 <= n) {
       *reinterpret_cast<uint2*>(y + i) =
-          make_uint2(e4m3_pair<BF16>(v[u].x) | (e4m3_pair<BF16>(v[u].y) << 16), e4m3_pair<BF16>(v[u].z) | (e4m3_pair<BF16>(v[u].w) << 16));
+          make_uint2(e4m3_pair<BF16>(v[u].x, limit) | (e4m3_pair<BF16>(v[u].y, limit) << 16), e4m3_pair<BF16>(v[u].z, limit) | (e4m3_pair<BF16>(v[u].w, limit) << 16));
     } else {
-      for (int64_t j = i; j < n; ++j) y[j] = static_cast<uint8_t>(e4m3_pair<BF16>(x[j]));
+      for (int64_t j = i; j < n; ++j) y[j] = static_cast<uint8_t>(e4m3_pair<BF16>(x[j], limit));
     }
   }
   pdl_launch_dependents();
@@ -293,14 +293,15 @@ static int launch_gated_unit(const void* x, void* y, int64_t rows, int cols, int
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
-extern "C" int ortb200_cast_e4m3(const void* x, void* y, int64_t n, int dtype, ortb200_stream_t stream_) {
+extern "C" int ortb200_cast_e4m3(const void* x, void* y, int64_t n, int dtype, int saturate, ortb200_stream_t stream_) {
   cudaStream_t st = static_cast<cudaStream_t>(stream_);
   if (!x || !y || n <= 0) return -1;
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(y) & 7)) return -3;
   const int64_t blocks = (n + 4095) / 4096;
   if (blocks > 0x7fffffff) return -9;
-  if (dtype == ORTB200_BF16) cast_e4m3_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n);
-  else if (dtype == ORTB200_F16) cast_e4m3_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n);
+  const float limit = saturate ? INFINITY : 464.f;
+  if (dtype == ORTB200_BF16) cast_e4m3_kernel<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n, limit);
+  else if (dtype == ORTB200_F16) cast_e4m3_kernel<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint16_t*>(x), static_cast<uint8_t*>(y), n, limit);
   else return -4;
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }

@@ -412,9 +412,9 @@ int64_t ortb200_argmax_workspace_bytes(int64_t rows);
 // y = act(x + bias[col]) elementwise; bias optional, cols = last dimension
 int ortb200_bias_act(const void* x, const void* bias, void* y, int64_t rows, int cols, int act, float alpha, int dtype,
                      ortb200_stream_t stream);
-// y (e4m3 bytes) = x (16-bit), rounded to nearest even; beyond 464 (where rounding passes the largest number, 448) and for
-// NaN: the NaN byte with the sign of x in 32 bits, as the tensor library converts.  x 16-byte and y 8-byte aligned.
-int ortb200_cast_e4m3(const void* x, void* y, int64_t n, int dtype, ortb200_stream_t stream);
+// y (e4m3 bytes) = x (16-bit), rounded to nearest even.  Beyond 464, where rounding passes the largest number: 448 with
+// `saturate`, else the NaN byte.  NaN: the NaN byte with the sign of x.  x 16-byte and y 8-byte aligned.
+int ortb200_cast_e4m3(const void* x, void* y, int64_t n, int dtype, int saturate, ortb200_stream_t stream);
 // y = act(gate) * up for x = [rows, 2 * cols] split in halves (gate | up): silu, or the tanh form of gelu (GEGLU)
 int ortb200_swiglu(const void* x, void* y, int64_t rows, int cols, int dtype, ortb200_stream_t stream);
 int ortb200_geglu(const void* x, void* y, int64_t rows, int cols, int dtype, ortb200_stream_t stream);
