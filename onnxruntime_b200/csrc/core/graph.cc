@@ -440,6 +440,7 @@ std::shared_ptr<Graph> Graph::FromProto(const pb::GraphProto& g, const std::map<
         for (auto& t : held.tensors) own(t);
       }
     }
+    for (auto& e : n.metadata_props) node->metadata[e.key] = e.value;
     node->since_version = static_cast<int>(out->Opset(node->domain));
   }
   return out;
@@ -463,6 +464,7 @@ pb::GraphProto Graph::ToProto() const {
       a.g = std::make_shared<pb::GraphProto>(kv.second->ToProto());
       np.attribute.push_back(std::move(a));
     }
+    for (auto& kv : n->metadata) np.metadata_props.push_back({kv.first, kv.second});
     g.node.push_back(std::move(np));
   }
   for (auto& kv : initializers_) {

@@ -45,6 +45,7 @@ struct Node {
   std::vector<std::string> inputs, outputs;  // "" marks an omitted optional
   std::map<std::string, pb::AttributeProto> attrs;
   std::map<std::string, std::shared_ptr<Graph>> subgraphs;  // attribute name -> body
+  std::map<std::string, std::string> metadata;              // NodeProto.metadata_props: other runtimes pass over what they do not know
   std::string ep;  // execution provider assigned by the partitioner
   int since_version = 0;
   bool removed = false;  // set by Graph::RemoveNode; the object lives on until Graph::PurgeRemoved()

@@ -840,7 +840,8 @@ class EmbedLayerNormKernel final : public WithFallback {
  public:
   explicit EmbedLayerNormKernel(const OpKernelInfo& info) : WithFallback(info) {
     eps_ = info.node.attr_f("epsilon", 1e-12f);
-    from_gathers_ = info.node.attr_i("ortb200_from_gathers", 0) != 0;
+    // (an attribute in models that were saved before nodes kept metadata)
+    from_gathers_ = info.node.metadata.count("ortb200.from_gathers") != 0 || info.node.attr_i("ortb200_from_gathers", 0) != 0;
   }
   void Compute(Ctx& ctx) const override {
     const at::Tensor& ids = ctx.RequiredInput(0);

@@ -487,7 +487,8 @@ int EmbedLayerNormFusion(PassContext& c) {
       const std::string mask_out = g.UniqueName("embed_mask_index");
       Node* f = g.AddNode("EmbedLayerNormalization", ins, {ln->outputs[0], mask_out}, kMSDomain, g.UniqueName("EmbedLayerNorm"));
       f->set_attr_f("epsilon", ln->attr_f("epsilon", 1e-12f));
-      if (derived) f->set_attr_i("ortb200_from_gathers", 1);   // the GPU kernel then reads ids as Gather does
+      // the GPU kernel then reads ids as Gather does; in the metadata, for the operator's schema has no such attribute
+      if (derived) f->metadata["ortb200.from_gathers"] = "1";
       g.RemoveNode(ln);
       for (Node* a : adds) g.RemoveNode(a);
       for (Node* ga : gathers) g.RemoveNode(ga);

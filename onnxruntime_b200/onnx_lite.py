@@ -183,6 +183,7 @@ class Node:
     name: str = ""
     domain: str = ""
     attributes: List[Attribute] = field(default_factory=list)
+    metadata: Dict[str, str] = field(default_factory=dict)
 
     def serialize(self) -> bytes:
         out = b"".join(_f_str(1, i) for i in self.inputs)
@@ -193,6 +194,8 @@ class Node:
         out += b"".join(_f_bytes(5, a.serialize()) for a in self.attributes)
         if self.domain:
             out += _f_str(7, self.domain)
+        for k, v in self.metadata.items():
+            out += _f_bytes(9, _f_str(1, k) + _f_str(2, v))
         return out
 
 
@@ -552,6 +555,9 @@ def _node_from_bytes(buf: bytes) -> Node:
             n.attributes.append(_attribute_from_bytes(v))
         elif f == 7:
             n.domain = bytes(v).decode()
+        elif f == 9:
+            kv = {ff: bytes(vv).decode() for ff, _, vv in parse_message(v)}
+            n.metadata[kv.get(1, "")] = kv.get(2, "")
     return n
 
 

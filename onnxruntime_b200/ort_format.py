@@ -32,6 +32,8 @@ _TS_ELEM, _TS_SHAPE = range(2)
 _DIM_VALUE, _DIM_DENOTATION = range(2)
 _DV_TYPE, _DV_VALUE, _DV_PARAM = range(3)
 
+_OWN = "ortb200."   # node metadata of this runtime: nodes of this format have none, so it travels as attributes of these names
+
 
 def is_ort_format(buf) -> bool:
     return len(buf) >= 8 and bytes(buf[4:8]) == IDENTIFIER
@@ -96,6 +98,9 @@ def _graph(g: fb.Table, name: str) -> ol.Graph:
     for n in sorted(g.tables(_G_NODES), key=lambda n: n.scalar(_N_INDEX, "I")):
         nodes.append(ol.Node(n.string(_N_OP), n.strings(_N_INPUTS), n.strings(_N_OUTPUTS), n.string(_N_NAME), n.string(_N_DOMAIN),
                              [_attribute(a) for a in n.tables(_N_ATTRS)]))
+        for a in [a for a in nodes[-1].attributes if a.name.startswith(_OWN)]:
+            nodes[-1].attributes.remove(a)
+            nodes[-1].metadata[a.name] = a.value.decode() if isinstance(a.value, bytes) else a.value
     in_names, out_names = g.strings(_G_INPUTS), g.strings(_G_OUTPUTS)
     take = lambda names: [infos.get(n, ol.ValueInfo(n)) for n in names]
     inner = set(in_names) | set(out_names)
@@ -175,9 +180,11 @@ def _w_graph(g: ol.Graph, opsets: Optional[Dict[str, int]] = None):
     infos = {v.name: v for v in list(g.value_info) + list(g.inputs) + list(g.outputs)}
     nodes = []
     for i, n in enumerate(g.nodes):
+        own = [ol.Attribute(k, ol.ATTR_STRING, v) for k, v in n.metadata.items() if k.startswith(_OWN)]
         since = (opsets or {}).get(n.domain if n.domain != "ai.onnx" else "", 0)
         nodes.append([("str", n.name), None, ("str", n.domain), ("i32", int(since)), ("u32", i), ("str", n.op_type), ("i32", 0), None,
-                      ("vec_str", list(n.inputs)), ("vec_str", list(n.outputs)), ("vec_table", [_w_attribute(a) for a in n.attributes])])
+                      ("vec_str", list(n.inputs)), ("vec_str", list(n.outputs)),
+                      ("vec_table", [_w_attribute(a) for a in n.attributes + own])])
     return [("vec_table", [_w_tensor(t) for t in g.initializers]), ("vec_table", [_w_value_info(v) for v in infos.values()]),
             ("vec_table", nodes), ("u32", max(len(g.nodes) - 1, 0)), None,
             ("vec_str", [v.name for v in g.inputs]), ("vec_str", [v.name for v in g.outputs])]
