@@ -41,14 +41,16 @@ constexpr int kUnit = 2;            // k-blocks per pipeline stage: one barrier 
 template <int BN>
 struct Q4Smem {
   static constexpr int kXBytes = BN * kBK * 2;         // activations of one k-block
-  static constexpr int kCtasPerSm = BN <= 8 ? 6 : 5;   // 64 and 72 registers
+  // Registers: 64 and, for 9 to 16 tokens, 72 in bf16.  In fp16 these spill, and four CTAs an SM (94 registers) are mostly faster
+  // (57344 x 8192, 16 tokens: 104 -> 100 us, 8192 x 28672 61 -> 57, 8192 x 8192 27 -> 25, but 10240 x 8192 31 -> 31.6).
+  static constexpr int ctas_per_sm(bool bf16) { return BN <= 8 ? 6 : bf16 ? 5 : 4; }
   static constexpr int kStages = 3;
   // activations first: their swizzle counts from 1 KiB boundaries
   static constexpr int kOffBlob = kUnit * kXBytes * kStages;
   static constexpr int kOffBar = kOffBlob + kUnit * kBlobBytes * kStages;
   static constexpr int kPartBytes = BN * kRows * 4;    // re-uses the drained stages
   static constexpr int kTotal = kOffBar + 16 * kStages + 1024;
-  static_assert(kPartBytes <= kOffBar && kTotal * kCtasPerSm <= 222 * 1024, "shared memory");
+  static_assert(kPartBytes <= kOffBar && kTotal * ctas_per_sm(true) <= 222 * 1024, "shared memory");
   static_assert(kOffBar % 8 == 0 && kOffBlob % 16 == 0, "alignment of barriers and bulk copies");
 };
 
@@ -109,7 +111,7 @@ __device__ __forceinline__ void mma_16x8x16(float (&c)[4], const uint32_t (&a)[4
 }
 
 template <int BN, bool BF16>
-__global__ void __launch_bounds__(kThreads, Q4Smem<BN>::kCtasPerSm)
+__global__ void __launch_bounds__(kThreads, Q4Smem<BN>::ctas_per_sm(BF16))
 gemm_q4_kernel(const __grid_constant__ CUtensorMap tmap_x, const SmallGemmParams p) {
   using S = Q4Smem<BN>;
   constexpr int STAGES = S::kStages, NT = BN / 8;
@@ -157,17 +159,19 @@ gemm_q4_kernel(const __grid_constant__ CUtensorMap tmap_x, const SmallGemmParams
       for (int i = 0; i < pre; ++i) load_w(i, i);
       pdl_wait_prior_grids();
       for (int i = 0; i < pre; ++i) load_x(i, i);
-      int s = 0;
+      int s = 0, issued = pre;
       uint32_t parity = 0;
-      for (int i = pre; i < nu; ++i) {
+      for (; issued < nu; ++issued) {
         if (!mbar_wait(&empty_bar[s], parity)) {
           if (p.status) atomicExch(p.status, kStatusTimeoutProducer);
           break;
         }
-        load_w(i, s);
-        load_x(i, s);
+        load_w(issued, s);
+        load_x(issued, s);
         if (++s == STAGES) { s = 0; parity ^= 1u; }
       }
+      // whoever gave up, no copy is in flight when this CTA leaves
+      for (int i = max(issued - STAGES, 0); i < issued; ++i) mbar_wait(&full_bar[i % STAGES], (i / STAGES) & 1);
     }
     __syncwarp();
   } else {
@@ -186,6 +190,7 @@ gemm_q4_kernel(const __grid_constant__ CUtensorMap tmap_x, const SmallGemmParams
     uint32_t parity = 0;
     for (int i = 0; i < nu; ++i) {
       if (ok && !mbar_wait(&full_bar[s], parity)) ok = false;
+      __syncwarp();   // the products are warp-wide, also where only some lanes gave up
       const int nb = min(kUnit, p.num_kb - (u_begin + i) * kUnit);
 #pragma unroll
       for (int k = 0; k < kUnit; ++k) {

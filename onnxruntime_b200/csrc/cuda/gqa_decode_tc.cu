@@ -170,7 +170,8 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // ------------------------------------------------------------ TMA producer (with a paged cache lane i fetches piece i)
     const int pieces = PAGED ? kTile / piece_rows : 1;
     bool ok = true;
-    for (int i = 0; i < 2 * n_tiles; ++i) {
+    int i = 0;
+    for (; i < 2 * n_tiles; ++i) {
       const int s = i % kSlots, key0 = k_begin + (i >> 1) * kTile;
       if (i >= kSlots && !mbar_wait_warp(&bars[BAR_EMPTY0 + s], ((i / kSlots) - 1) & 1)) { ok = false; break; }
       uint8_t* dst = smem + s * kTileBytes;
@@ -199,6 +200,8 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       __syncwarp();
     }
+    // whoever gave up, no copy is in flight when the slots serve the merge or the CTA leaves
+    for (int j = max(i - kSlots, 0); j < i; ++j) ok = mbar_wait_warp(&bars[BAR_FULL0 + j % kSlots], (j / kSlots) & 1) && ok;
     if (!ok && lane == 0 && p.status) atomicExch(p.status, kStatusTimeoutProducer);
   } else if (warp == 4) {
     // ------------------------------------------------------------ MMA issuer: the whole warp waits, lane 0 issues (a lone
@@ -351,7 +354,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // A wait that gives up clears `ok`; the loop still runs to its end (without further waits) so that every
     // thread keeps meeting the others at the named barrier and publishes P for the MMA warp.
     for (int t = 0; t < n_tiles; ++t) {
-      if (ok && !mbar_wait(&bars[BAR_S0 + (t & 1)], (t >> 1) & 1)) ok = false;
+      if (ok && !mbar_wait_warp(&bars[BAR_S0 + (t & 1)], (t >> 1) & 1)) ok = false;
       tcgen05_fence_after();
       float sv[GV];
       tmem_ld_heads<G>(tmem_base + lane_addr + (t & 1) * 16, sv);
@@ -385,7 +388,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int g = 0; g < G; ++g) l_part[g] *= corr[g];
         if (t > 0) {
           // O^T holds the sum up to tile t - 1 once its MMA has finished; thread t rescales its dim
-          if (ok && !mbar_wait(&bars[BAR_O], (t - 1) & 1)) ok = false;
+          if (ok && !mbar_wait_warp(&bars[BAR_O], (t - 1) & 1)) ok = false;
           tcgen05_fence_after();
           float ov[GV];
           tmem_ld_heads<G>(tmem_o + lane_addr, ov);
@@ -418,7 +421,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (k_begin + (t + 1) * kTile > k_end) {
         // last, partial tile: rows past the range hold whatever the cache (or an earlier tile) left there; a
         // non-finite value times a zero probability would poison MMA 2, so those V rows are cleared
-        if (ok && !mbar_wait(&bars[BAR_FULL0 + (2 * t + 1) % kSlots], ((2 * t + 1) / kSlots) & 1)) ok = false;
+        if (ok && !mbar_wait_warp(&bars[BAR_FULL0 + (2 * t + 1) % kSlots], ((2 * t + 1) / kSlots) & 1)) ok = false;
         if (!valid) {
           uint8_t* vrow = smem + ((2 * t + 1) % kSlots) * kTileBytes + tid * 128;
 #pragma unroll
@@ -447,7 +450,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   }
   if (warp < 4 && ok && n_tiles > 0) {
     // a barrier of its own: the product of tile n - 2 may still run, and BAR_O's parity would then read as done
-    if (!mbar_wait(&bars[BAR_END], 0)) {
+    if (!mbar_wait_warp(&bars[BAR_END], 0)) {
       ok = false;
       if (p.status) atomicExch(p.status, kStatusTimeoutEpilogue);
     }
