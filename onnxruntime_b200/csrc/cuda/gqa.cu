@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(128) gqa_decode_kernel(const DecodeParams p) {
     fa[g] = aa;
   }
 
-  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last, sm_acc);
+  decode_finish<T, H, G>(p, tile, split, p.splits, b, head0, n_heads, tid, fm, fl, fa, &sm_last, sm_acc);
 }
 
 

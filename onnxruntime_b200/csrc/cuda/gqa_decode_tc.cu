@@ -23,6 +23,7 @@
 // flash-decoding path (bert/flash_attention/flash_api.cc, mha_fwd_kvcache) and PagedDecodeSplitKV
 // (bert/paged_attention_impl.cu).
 #include <cuda.h>
+#include <algorithm>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <type_traits>
@@ -43,9 +44,9 @@ constexpr int kMaxSlots = 6;
 constexpr int kSms = 148;
 // K and V tiles alternate through one ring of slots.  Six slots: one CTA per SM, for grids that fit the machine once.  Three
 // slots: two CTAs share an SM with the same bytes in flight, and one's prologue, query rotation and merge of splits run while
-// the other streams.  40 sequences of 1000 - 4000 keys, 8 kv heads of 128, bf16: 101 -> 82 us (the bytes need 60); 32 of 1024 -
-// 4096, 8 heads per kv head: 90 -> 74 (47); one of 4096 in 16 splits: 30 -> 15 (mostly the merge).  (The remainders of SPLIT
-// take shared memory: always six.)
+// the other streams.  40 sequences of 1000 - 4000 keys, 8 kv heads of 128, bf16, take 82 us with three slots and the merge by all
+// threads, 101 with three stages of K and V and a merge by one (the bytes need 60); 32 of 1024 - 4096, 8 heads per kv head, 74
+// and 90 (47); one of 4096 in 16 splits 15 and 30 (mostly the merge).  (The remainders of SPLIT take shared memory: always six.)
 template <bool SPLIT, int SLOTS>
 struct Smem {
   static constexpr int kSlots = SLOTS;
@@ -89,6 +90,33 @@ __device__ __forceinline__ void tmem_ld_heads(uint32_t taddr, float* v) {
   tmem_ld_wait();
 }
 
+// Keys of sequence b: positions [first, total), of which the tiles start at `start`; `splits` of the launched ones share them.
+struct KeyRange {
+  int total, first, start, len, splits;
+};
+template <bool PAGED>
+__device__ __forceinline__ KeyRange key_range(const DecodeParams& p, int b, int piece_rows) {
+  KeyRange r;
+  r.total = max(min(p.seqlens_k[b] + 1, p.Smax), 0);
+  r.first = p.window > 0 ? max(0, r.total - p.window) : 0;
+  if (p.chunk > 0) r.first = max(r.first, (r.total - 1) / p.chunk * p.chunk);
+  r.start = PAGED ? r.first / piece_rows * piece_rows : r.first;   // tiles start on piece boundaries
+  r.len = max(r.total - r.start, 0);
+  r.splits = p.piece_tiles > 0 ? min(p.splits, max(1, r.len / (p.piece_tiles * kTile))) : p.splits;
+  return r;
+}
+// Asks the L2 for this CTA's slice of the next kernel's weights (a grid moves a few tens of MB and leaves most of the memory
+// bandwidth idle).  One warp.
+__device__ __forceinline__ void prefetch_slice(const DecodeParams& p, int lane) {
+  const long long cta = (static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const long long lo = cta * p.prefetch_per_cta;
+  const long long hi = lo + p.prefetch_per_cta < p.prefetch_bytes ? lo + p.prefetch_per_cta : p.prefetch_bytes;
+  for (long long off = lo + static_cast<long long>(lane) * 16384; off < hi; off += 32 * 16384) {
+    const long long nbytes = hi - off < 16384 ? hi - off : 16384;
+    bulk_prefetch_l2(p.prefetch + off, static_cast<uint32_t>(nbytes));
+  }
+}
+
 template <typename T, int G, bool PAGED, bool SPLIT, int SLOTS>
 __global__ void __launch_bounds__(kThreads, SLOTS == 3 ? 2 : 1)
 gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -113,10 +141,18 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const bool fused = p.qkv != nullptr;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int kvh = blockIdx.x, split = p.splits_last ? blockIdx.z : blockIdx.y, b = p.splits_last ? blockIdx.y : blockIdx.z;
   const int group = p.N / p.Nk;
   const int head0 = kvh * group;
   const int n_heads = group;
+  if (p.piece_tiles > 0 && split > 0) {
+    // the grid has room for the longest sequence: what a shorter one does not need leaves before it takes anything
+    pdl_wait_prior_grids();
+    if (split >= key_range<PAGED>(p, b, piece_rows).splits) {
+      if (warp == 5 && p.prefetch != nullptr) prefetch_slice(p, lane);
+      return;
+    }
+  }
 
   if (tid == 0) {
     tma_prefetch_desc(&tm_q);
@@ -136,17 +172,11 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const uint32_t tmem_o = tmem_base + 32;
 
   pdl_wait_prior_grids();
-  int total = p.seqlens_k[b] + 1;
-  if (total > p.Smax || total < 0) {
-    // a length beyond the cache capacity would read past the buffer: attend to what the cache holds and report it
-    if (threadIdx.x == 0 && p.status) atomicExch(p.status, kStatusBadLength);
-    total = total < 0 ? 0 : p.Smax;
-  }
-  int first_key = p.window > 0 ? max(0, total - p.window) : 0;
-  if (p.chunk > 0) first_key = max(first_key, (total - 1) / p.chunk * p.chunk);
-  const int start0 = PAGED ? first_key / piece_rows * piece_rows : first_key;   // tiles start on piece boundaries
-  const int len = max(total - start0, 0);
-  int chunk = (len + p.splits - 1) / p.splits;
+  const KeyRange keys = key_range<PAGED>(p, b, piece_rows);
+  const int total = keys.total, first_key = keys.first, start0 = keys.start, splits = keys.splits;
+  // a length beyond the cache capacity would read past the buffer: attend to what the cache holds and report it
+  if (threadIdx.x == 0 && p.status && p.seqlens_k[b] + 1 != total) atomicExch(p.status, kStatusBadLength);
+  int chunk = (keys.len + splits - 1) / splits;
   if (PAGED) chunk = (chunk + kTile - 1) / kTile * kTile;
   const int k_begin = start0 + split * chunk;
   // fused: the newest key (position total - 1) is not in the cache yet; the CTA whose range reaches it takes it
@@ -154,17 +184,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int k_end = owns_new ? total - 1 : min(total, k_begin + chunk);
   const int n_tiles = k_end > k_begin ? (k_end - k_begin + kTile - 1) / kTile : 0;
 
-  if (warp == 5 && p.prefetch != nullptr) {
-    // This grid moves a few tens of MB and leaves most of the memory bandwidth idle: ask the L2 for this CTA's slice
-    // of the next kernel's weights now, so that kernel finds them on chip.
-    const long long cta = (static_cast<long long>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    const long long lo = cta * p.prefetch_per_cta;
-    const long long hi = lo + p.prefetch_per_cta < p.prefetch_bytes ? lo + p.prefetch_per_cta : p.prefetch_bytes;
-    for (long long off = lo + static_cast<long long>(lane) * 16384; off < hi; off += 32 * 16384) {
-      const long long nbytes = hi - off < 16384 ? hi - off : 16384;
-      bulk_prefetch_l2(p.prefetch + off, static_cast<uint32_t>(nbytes));
-    }
-  }
+  if (warp == 5 && p.prefetch != nullptr) prefetch_slice(p, lane);
   // load i is the K tile (i even) or the V tile (i odd) of key tile i / 2, in slot i % kSlots
   if (warp == 5) {
     // ------------------------------------------------------------ TMA producer (with a paged cache lane i fetches piece i)
@@ -502,7 +522,7 @@ gqa_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
   }
   const int tile = b * p.Nk + kvh;
-  decode_finish<T, H, G>(p, tile, split, b, head0, n_heads, tid, fm, fl, fa, &sm_last, reinterpret_cast<float*>(smem));
+  decode_finish<T, H, G>(p, tile, split, splits, b, head0, n_heads, tid, fm, fl, fa, &sm_last, reinterpret_cast<float*>(smem));
 }
 
 template <typename T, int G, bool PAGED, bool SPLIT, int SLOTS>
@@ -575,19 +595,24 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   const int group = a->N / a->Nk;
   const int G = group <= 4 ? 4 : (group <= 8 ? 8 : 16);
   const int base = a->B * a->Nk;
-  int splits = a->splits;
+  int splits = a->splits, piece_tiles = 0;
   if (splits <= 0) {
     // Small grids: one CTA per SM at most.  Merging splits costs about as much as four tiles, so a grid that already covers a
     // good part of the machine with short key ranges is not split; otherwise at least two tiles per split.
-    // Grids of more than half the machine: two or three splits of at least ten tiles even out unequal lengths (20 sequences of
-    // 750 - 3000 keys, 8 kv heads: 51 us in one piece, 41 in two; 40 of 1000 - 4000: 87 and, in three, 82; 64 of 250 - 1000
-    // would lose, 43 and 51).
+    // Grids of more than half the machine: up to three splits even out unequal lengths.  The capacity of a cache says nothing of
+    // the lengths, so each sequence takes a split per piece_tiles tiles of its keys and the other CTAs leave at once; the
+    // fuller the machine is without them, the longer a split has to be to be worth its merge.  Windows make lengths equal: one
+    // split.  8 kv heads, room for 8192 keys, lengths from a quarter to all of the number, us with one split / three whatever
+    // the length / this rule: 20 sequences of 1500 keys 32 / 28.7 / 29.3, 20 of 3000 56 / 42.9 / 43.1, 25 of 4000 73 / 59 / 59,
+    // 40 of 4000 90 / 84 / 83, 64 of 1000 44 / 56 / 44, 64 of 2500 - / 93 / 88, 48 of 200 each 21 / 34 / 21.5; 20 with a
+    // window of 128 keys 7.4 / 22 / 7.4, of 1024 22.5 / 29 / 22.5.
     // a chunk may begin within a tile
     const int tiles = a->chunk > 0 && a->chunk < a->Smax - kTile ? (a->chunk + kTile - 1) / kTile + 1 : (a->Smax + kTile - 1) / kTile;
     if (base >= 32 && tiles <= 12) {
       splits = 1;
     } else if (base > kSms / 2) {
-      splits = tiles >= 30 ? 3 : tiles >= 20 ? 2 : 1;
+      piece_tiles = std::max(2, base / 64);
+      splits = a->window > 0 && a->window < a->Smax ? 1 : std::max(1, std::min(3, tiles / piece_tiles));
     } else {
       splits = kSms / base;
       if (splits > (tiles + 1) / 2) splits = (tiles + 1) / 2;
@@ -634,7 +659,11 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream) 
   p.block_table = a->block_table; p.block_size = a->block_size; p.max_blocks = a->max_blocks;
   p.qkv = a->qkv; p.cos_cache = a->cos_cache; p.sin_cache = a->sin_cache; p.cos_rows = a->cos_rows;
   p.do_rotary = a->do_rotary; p.interleaved = a->rotary_interleaved;
-  dim3 grid(splits, a->Nk, a->B);
+  p.piece_tiles = piece_tiles;
+  // The splits of a sequence side by side; but where the first splits alone more than fill the machine, those come first, and
+  // CTAs that leave cost nothing (48 sequences of 200 keys: 22.6 and 21.4 us; 40 of 1000 - 4000 side by side 82, else 85).
+  p.splits_last = piece_tiles > 0 && base > 2 * kSms * 5 / 4;
+  const dim3 grid = p.splits_last ? dim3(a->Nk, a->B, splits) : dim3(a->Nk, splits, a->B);
   p.chunk = a->chunk;
   p.q_ld = q_ld;
   p.out_ld = a->out_ld > 0 ? a->out_ld : static_cast<long long>(a->N) * H;

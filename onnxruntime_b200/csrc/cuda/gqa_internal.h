@@ -18,6 +18,8 @@ struct DecodeParams {
   unsigned int* counters;
   int* status;
   int B, N, Nk, Smax, splits, window, gparts;
+  int splits_last;         // (tcgen05 kernel) order of the grid: splits outermost instead of sequences
+  int piece_tiles;         // > 0 (tcgen05 kernel): a sequence uses a split per this many tiles of its keys, at most `splits`
   float scale, softcap;
   // paged cache [num_blocks, block_size, Nk, H]: key j of sequence b lives in block block_table[b, j / block_size]
   const int* block_table;
@@ -59,19 +61,20 @@ int launch_gqa_decode_tc(const ortb200_gqa_decode_args* a, cudaStream_t stream);
 
 // Tail of a decode-attention CTA.  On entry thread tid < H holds, for each of the G query heads, its dim of the
 // unnormalised output (fa), and every thread holds the running maximum (fm, natural-log domain) and the sum of
-// exponentials (fl) of the CTA's key range.  With splits > 1 the state goes to the workspace and the CTA that
-// arrives last on the tile's counter merges all splits; that CTA (or the only one) normalises and stores.
+// exponentials (fl) of the CTA's key range.  With splits > 1 (of this sequence: at most p.splits) the state goes to the
+// workspace and the CTA that arrives last on the tile's counter merges all splits; that CTA (or the only one) normalises and
+// stores.
 // `scratch`: 2 * splits * G floats of shared memory that nothing else needs any more.  In the merge a thread owns four dims of
 // one head and fetches eight splits at a time, after all threads have fetched the maxima and sums: a dim per thread, head
 // after head and load after load, was a chain of 2 * splits * G L2 round trips.
 template <typename T, int H, int G>
-__device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, int split, int b, int head0, int n_heads,
+__device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, int split, int splits, int b, int head0, int n_heads,
                                               int tid, float (&fm)[G], float (&fl)[G], float (&fa)[G],
                                               unsigned int* sm_last_ptr, float* scratch) {
   const bool owner = tid < H;
   unsigned int& sm_last = *sm_last_ptr;
   bool finalize = true;
-  if (p.splits > 1) {
+  if (splits > 1) {
     // publish partial state: ws[tile][split][g][H + 4]
     constexpr int kState = H + 4;   // rows of 16-byte vectors
     float* my = p.ws + ((static_cast<size_t>(tile) * p.splits + split) * G) * kState;
@@ -87,7 +90,7 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, i
     __syncthreads();
     if (tid == 0) {
       const unsigned int old = atomicAdd(&p.counters[tile], 1u);
-      const unsigned int last = old == static_cast<unsigned int>(p.splits - 1) ? 1u : 0u;
+      const unsigned int last = old == static_cast<unsigned int>(splits - 1) ? 1u : 0u;
       if (last) p.counters[tile] = 0;
       sm_last = last;
     }
@@ -96,7 +99,7 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, i
     if (sm_last != 0) {
       __threadfence();
       const float* base = p.ws + (static_cast<size_t>(tile) * p.splits * G) * kState;
-      const int states = p.splits * G;
+      const int states = splits * G;
       for (int i = tid; i < states; i += blockDim.x) {
         scratch[i] = __ldcg(&base[i * kState + H]);
         scratch[states + i] = __ldcg(&base[i * kState + H + 1]);
@@ -105,16 +108,16 @@ __device__ __forceinline__ void decode_finish(const DecodeParams& p, int tile, i
       for (int i = tid; i < n_heads * (H / 4); i += blockDim.x) {
         const int g = i / (H / 4), d = i % (H / 4) * 4;
         float mm = kNegBig;
-        for (int s = 0; s < p.splits; ++s) mm = fmaxf(mm, scratch[s * G + g]);
+        for (int s = 0; s < splits; ++s) mm = fmaxf(mm, scratch[s * G + g]);
         float ll = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int s0 = 0; s0 < p.splits; s0 += 8) {
+        for (int s0 = 0; s0 < splits; s0 += 8) {
           float4 v[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            v[e] = s0 + e < p.splits ? __ldcg(reinterpret_cast<const float4*>(&base[((s0 + e) * G + g) * kState + d])) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[e] = s0 + e < splits ? __ldcg(reinterpret_cast<const float4*>(&base[((s0 + e) * G + g) * kState + d])) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            if (s0 + e >= p.splits) break;
+            if (s0 + e >= splits) break;
             const float c = safe_exp_diff(scratch[(s0 + e) * G + g], mm);
             ll += scratch[states + (s0 + e) * G + g] * c;
             acc[0] += v[e].x * c;
