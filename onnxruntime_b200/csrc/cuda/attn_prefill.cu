@@ -11,9 +11,9 @@
 // The bound is the exponentials (16 a clock and SM: 512 clocks a tile) and the latency of the chain S -> softmax -> P V.
 // P takes no shared memory and S / P two buffers of 64 columns, so two CTAs share an SM (256 columns, at most 98 KB each):
 // one's chain, prologue and epilogue hide behind the other's.
-// Against one CTA per SM with 128-key tiles, P in shared memory and one query head per CTA: 8 x 1024 causal, 32 / 8 heads of
-// 128: 250 -> 122 us; 64 x 384 masked, 16 heads of 64: 286 -> 115 us; 2284 packed tokens of 25 sequences, 20 of them single
-// tokens: 206 -> 91 us.  2 x 4096 causal reaches 877 TFLOP/s; at 8 x 1024 (9 tiles a CTA) the special-function units are
+// 8 x 1024 causal, 32 / 8 heads of 128, takes 125 us so and 250 with one CTA per SM, 128-key tiles, P in shared memory and one
+// query head per CTA; 64 x 384 masked, 16 heads of 64, 116 and 286; 2284 packed tokens of 25 sequences, 20 of them single
+// tokens, 91 and 206.  2 x 4096 causal reaches 877 TFLOP/s; at 8 x 1024 (9 tiles a CTA) the special-function units are
 // 31 % busy: what is left is the latency of a CTA's first loads and last stores.
 // Value rows behind the last visible key (of a cache, or of a masked tail) may hold anything and never reach the product.  Rows
 // that a key mask hides in front of that key take part with weight 0 and have to be finite.

@@ -91,9 +91,10 @@ struct Smem2 {
 
 // Order in which the tiles are worked on: runs of up to kRunTiles token tiles, inside a run token tile first and weight
 // tile second, so that the pairs at work share few operand tiles and L2 serves the repeats.  With all token tiles in one
-// run (the order before this one) every weight tile streamed the whole activation matrix again: the 134 MB of 16384 routed
-// rows x 4096 do not fit the L2.  Mixture of experts over 8192 tokens: 5945 -> 4616 us with this order and the gated
-// epilogue; four layers of an 8B decoder over 8192 tokens: 13698 -> 12160 us.  In grouped mode a run never mixes experts, so each expert's weights are read about once.
+// run every weight tile would stream the whole activation matrix again, and the 134 MB of 16384 routed rows x 4096 do not
+// fit the L2.  A mixture of experts over 8192 tokens takes 4616 us with runs of ten and the gated epilogue and 5945 without
+// either, four layers of an 8B decoder over 8192 tokens 12160 and 13698.  In grouped mode a run never mixes experts, so each
+// expert's weights are read about once.
 struct TileOrder {
   int tiles_m, tiles_n, run;
   const int* starts;   // grouped mode: first token tile of every run, [runs + 1] (shared memory); null = uniform runs
@@ -336,8 +337,8 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   } else {
     // ---------------------------------------------------------------- epilogue: this CTA's 128 weight rows x 256 tokens
     // Two groups of four warps, each for half of the tokens with a staging buffer of its own: one group's global stores
-    // overlap the other's tensor-memory reads.  (One group that read while a second only helped with the stores left the
-    // epilogue longer than the main loop of 16 k-blocks: 24576 x 4096 x 1024 with GELU ran at 810 TFLOP/s.)
+    // overlap the other's tensor-memory reads.  (With one group that reads and a second that only helps with the stores the
+    // epilogue is longer than the main loop of 16 k-blocks: 24576 x 4096 x 1024 with GELU runs at 810 TFLOP/s.)
     const int group = (warp - 2) >> 2;
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     const int r = q * 32 + lane;

@@ -11,10 +11,10 @@
 // weights per row and two 16-byte loads of activations per token, all without bank conflicts.  The bound is the instruction
 // stream (about 200 per warp and 32 x 64 weights at 8 tokens), not the bandwidth.
 //
-// Measured against it (fp16, event-timed alone, L2 cold, launch included): 57344 x 8192 118 -> 85 us for one token, 123 -> 101
-// for 16; 8192 x 28672 58 -> 52 and 59 -> 61; 10240 x 8192 38 -> 27 and 40 -> 31; 28672 x 4096 39 -> 33 and 42 -> 39;
-// 4096 x 4096 15.5 -> 12.7 and 15.5 -> 14.3.  With 32 tokens the products cost more than the round trip saves (134 -> 138 and
-// 63 -> 80 us), so the tcgen05 form keeps everything above 16.
+// The two forms, tcgen05 / this, us for one and for 16 tokens (fp16, event-timed alone, L2 cold, launch included): 57344 x 8192
+// 118 / 86 and 123 / 100; 8192 x 28672 58 / 52 and 59 / 57; 10240 x 8192 38 / 27 and 40 / 31.6; 28672 x 4096 39 / 33 and 42 / 39;
+// 4096 x 4096 15.5 / 13 and 15.5 / 15.  With 32 tokens the products cost more than the round trip saves (134 / 138 and
+// 63 / 80 us), so the tcgen05 form keeps everything above 16.
 //
 // A cluster of C CTAs shares one 128-row tile over K and adds its partial tiles through distributed shared memory in rank
 // order, as in gemm_smallm.cu.

@@ -420,8 +420,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       // rows (a few KiB, L2 resident) and leave the factors in shared memory for the epilogue.
       pdl_wait_prior_grids();
       const int vecs = p.K / 8;
-      // Only the token columns that this CTA finishes: every CTA of the cluster used to read all rows (40 tokens x 4096:
-      // 47 us for the qkv projection of 50 MB).  Eight loads per lane go out before the first is used.
+      // Only the token columns that this CTA finishes (if every CTA of the cluster reads all rows, 40 tokens x 4096, the qkv
+      // projection of 50 MB takes 47 us).  Eight loads per lane go out before the first is used.
       for (int j = rank * (BN / C) + q; j < (rank + 1) * (BN / C); j += 4) {
         const int m = m0 + j;
         float ss = 0.f;
